@@ -449,7 +449,7 @@ int cct_ragged_plan_create(int32_t method, int32_t bp_mode, int32_t n_groups, co
     const int64_t per_slice = bands * d->n_angles * d->n_det;
     res[g] = cct::ResidualGroup{st->partials, per_slice, st->residuals, st->active, st->iterations, st->tolerance,
                                 st->residual_history, st->history_len};
-    const int64_t tiles = (int64_t)((d->n + 31) / 32) * ((d->n + 63) / 64);
+    const int64_t tiles = cct::bp_tile_count(d->n);
     fps[g + 1] = fps[g] + per_slice * d->n_slices;
     bps[g + 1] = bps[g] + tiles * d->n_slices;
     rss[g + 1] = rss[g] + d->n_slices;

@@ -13,13 +13,12 @@
 // The map of every angle is read from HBM once; the volume is L2-resident.
 //
 // Back projection (scikit-image iradon, filter None, corrct:
-// src/corrct/_projector_backends.py:335-359): one CTA owns a 32x32 pixel tile and
-// loops over all (detector, angle) lines in chunks of 32; each chunk stages, per
-// line, the <= 48 detector bins the tile can reach as (value, slope) pairs, and
-// every pixel does one shared-memory lookup and one FMA per line.  np.interp's
-// left=0 / right=0 edges are discontinuous, so lines whose range comes within
-// 0.01 bin of an edge take a checked path that decides edge cases in double
-// precision exactly as numpy does.
+// src/corrct/_projector_backends.py:335-359): one CTA owns a tile of 32 columns and 32 or
+// 64 rows and walks its (detector, angle) lines in chunks of 16; each chunk stages, per
+// line, the <= 74 detector bins the tile can reach as (value, slope) pairs, and every
+// pixel does one shared-memory lookup and one FMA per line.  np.interp's left=0 / right=0
+// edges are discontinuous: pixels within 0.01 bin of a detector edge are decided apart,
+// exactly as numpy decides them in double.
 
 #include <cstring>
 
@@ -795,188 +794,384 @@ __global__ void __launch_bounds__(FP_THREADS, 4) fp_pair_kernel(FpArgs args) {
 
 // ------------------------------------------------------------------------------------------
 // Back projection (reference iradon discretisation, optional maps x weights)
+//
+// A CTA owns a 32-column tile of TI = 32 or 64 rows; a warp holds TI / 8 whole rows of it.
+//
+// Bound: an 8-byte lookup is two shared-memory wavefronts whatever the lanes' pixels (0.40 ms of
+// them for 8 slices of 512^2 x 720), next the ~8 instructions per pixel and line.  What else
+// the time went on was the rare case: the FP64 edge decision, inlined per pixel or called, cost
+// registers and branches on every line (1.20 ms with the call, 0.99 ms with no edge at all, 1.13 ms
+// as below, for 16 slices), and the three barriers per chunk of lines.  Measured on 512^2 x 720
+// (start -> now): 1 slice 281 -> 106 us, 8 slices 880 -> 597 us, 16 slices 1519 -> 1128 us; 256^2 x
+// 360 161 -> 23 us, 128^2 x 180 77 -> 11 us; with maps (512^2 x 360, 2 slices) 1577 -> 278 us.
+//
+// The lines are summed in up to eight fixed segments, whose sums are added in order (which also
+// shortens the FP32 sums: the error against FP64 falls from 3.9e-7 to 1e-7 at 722 lines).  One CTA
+// walks all of them, or, where the batch has few tiles, the CTAs of a cluster take one each and
+// combine them through distributed shared memory; both give the same bits.
 // ------------------------------------------------------------------------------------------
-constexpr int BP_TJ = 32;                                // tile columns (one per lane)
-constexpr int BP_TI = 64;                                // tile rows
+constexpr int BP_TJ = 32;                                // tile columns
 constexpr int BP_THREADS = 256;
-constexpr int BP_PPT = BP_TI / (BP_THREADS / 32);        // 8 pixels (rows warp, warp+8, ...) per thread
-constexpr int BP_LINES = 32;                             // lines staged per chunk
+constexpr int BP_LINES = 16;                             // lines staged per chunk
 constexpr int BP_KW = 80;                                // staged pairs per line (>= 74 needed)
 constexpr float BP_EDGE_GUARD = 0.01f;
 
 enum : int { LINE_FAST = 0, LINE_CHECKED = 1, LINE_EMPTY = 2 };
 
-// One CTA of the back projection: pixel tile `tile` of slice `s`.
-template <int EPI, bool SYM, int MAPS_DTYPE>
-__device__ __forceinline__ void bp_cta(const BpArgs& args, const int tile, const int s) {
-  __shared__ __align__(16) float2 pairs[BP_LINES][BP_KW];
-  __shared__ float4 linfo[BP_LINES];  // cos, sin, offset (K - kbase), weight
-  __shared__ int lkind[BP_LINES];
-  __shared__ int lkbase[BP_LINES];
-  __shared__ float2 linner[BP_LINES];  // checked lines: interior range of the FP32 coordinate
+// Rows of a tile: small images take smaller tiles for more CTAs.  (The rounding of a pixel's bin
+// depends on its tile, so the choice depends on n alone.)
+__host__ __device__ inline int bp_tile_rows(int n) { return n > 192 ? 64 : 32; }
+__host__ __device__ inline int bp_tiles(int n) {
+  const int ti = bp_tile_rows(n);
+  return ((n + BP_TJ - 1) / BP_TJ) * ((n + ti - 1) / ti);
+}
+// log2 of the segments of the line sum (at least eight lines each); segment g of n_lines <= 65535
+// lines starts at (g * n_lines) >> log2.
+__host__ __device__ inline int bp_log2_segments(int n_lines) {
+  return n_lines >= 64 ? 3 : n_lines >= 32 ? 2 : n_lines >= 16 ? 1 : 0;
+}
 
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The float at shared address p of this CTA's layout in CTA `rank` of the cluster.
+__device__ __forceinline__ float cluster_load(const float* p, int rank) {
+  uint32_t a;
+  float v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+
+struct __align__(16) BpLine {
+  float cs, sn, off;      // cos, sin, K - kbase
+  int kind;
+  float mid, half;        // centre and half length of the detector in bins from kbase
+  float w;                // weight of the line
+  int kbase;
+};
+
+struct BpShared {
+  float2 pairs[2][BP_LINES][BP_KW];  // chunk being looked up, chunk being staged
+  BpLine line[3][BP_LINES];          // and the chunk after those
+};
+
+// np.interp(t, k - K, line, left=0, right=0) for a pixel (jc, ic from the centre) whose FP32 position
+// is within BP_EDGE_GUARD of a detector edge.  numpy decides the edge on t = jc cos - ic sin in
+// double, where both products are exact; here the distance d past the edge is formed from the
+// products' FP32 halves, the exact error of their difference and a difference with the edge that
+// is exact too (Sterbenz), so that only the last sum rounds: at |d| < 0.02 by less than 1e-11, with the
+// sign of a d that is exactly 0 (angles of 0 and 90 degrees) intact.  bins points at the staged
+// pair of bin 0.
+__device__ __forceinline__ float bp_edge_value(const float2* bins, float cs, float sn, int n, float jc, float ic) {
+  const int K = n / 2;
+  const float p = jc * cs, pe = fmaf(jc, cs, -p);
+  const float q = -ic * sn, qe = fmaf(-ic, sn, -q);
+  const float s = p + q, b = s - p;
+  const float se = (p - (s - b)) + (q - b);  // p + q = s + se exactly
+  const bool left = s < -0.5f;
+  const float d = (s + (left ? (float)K : -(float)(n - 1 - K))) + (se + (pe + qe));
+  if (left ? d < 0.f : d > 0.f) return 0.f;
+  const float2 v = bins[left ? 0 : n - 2];
+  return fmaf(left ? d : 1.f + d, v.y, v.x);
+}
+
+// Values of a staged line at two positions (bins from kbase), in packed FP32x2 arithmetic that rounds
+// like floor_split; `row` is the byte offset of the line's bin 0 in pairs, less the exponent bits
+// of the floors.
+__device__ __forceinline__ float2 bp_lerp2(const float2 (*pairs)[BP_KW], unsigned row, float2 u) {
+  const float2 magic = make_float2(12582912.0f, 12582912.0f);  // 1.5 * 2^23, see floor_split
+  const float2 nmagic = make_float2(-12582912.0f, -12582912.0f);
+  const float2 t = __fadd2_rd(u, magic);
+  const float2 f = __ffma2_rn(__fadd2_rn(t, nmagic), make_float2(-1.f, -1.f), u);  // u - floor(u), exact
+  const char* base = reinterpret_cast<const char*>(pairs);
+  const float2 p0 = *reinterpret_cast<const float2*>(base + ((__float_as_uint(t.x) << 3) + row));
+  const float2 p1 = *reinterpret_cast<const float2*>(base + ((__float_as_uint(t.y) << 3) + row));
+  return make_float2(fmaf(f.x, p0.y, p0.x), fmaf(f.y, p1.y, p1.x));
+}
+
+// Sum of lines [l0, l1) at the PPT pixels (rows i0 + k, column j) of this thread; ti0, tj0 is the
+// tile's first row and column.
+template <bool SYM, int MAPS_DTYPE, int PPT>
+__device__ __forceinline__ void bp_segment(const BpArgs& args, BpShared& sh, int s, int ti0, int tj0, int i0, int j,
+                                           int l0, int l1, float (&acc)[PPT]) {
+  static_assert(PPT % 2 == 0 && BP_LINES <= 32, "pixels go in pairs, lines in one mask");
+  constexpr int TI = 8 * PPT;
   const int n = args.n;
-  if (args.active != nullptr && args.active[s] == 0) return;
-  const int tiles_j = (n + BP_TJ - 1) / BP_TJ;
-  const int ti = tile / tiles_j;
-  const int tj = tile - ti * tiles_j;
-  const int i0 = ti * BP_TI, j0 = tj * BP_TJ;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int j = j0 + lane;
-  const int R = n / 2;      // iradon output radius (output_size // 2)
-  const int K = n / 2;      // detector offset (img_shape // 2)
-  const float t_left = (float)(-K), t_right = (float)(n - 1 - K);
-  const int n_lines = args.n_det * args.n_angles;
-  const float* sino = args.sino + (int64_t)s * n_lines * n;
+  const int K = n / 2;  // detector offset (img_shape // 2) and output radius (output_size // 2)
+  const float* sino = args.sino + (int64_t)s * args.n_det * args.n_angles * n;
+  const float fj = (float)(j - K);
+  float2 nfi[PPT / 2];
+  int pix[PPT];  // SYM: map offsets of the pixels (clamped into the image)
+#pragma unroll
+  for (int k = 0; k < PPT; ++k) {
+    const float v = -(float)(i0 + k - K);
+    if (k & 1) nfi[k / 2].y = v; else nfi[k / 2].x = v;
+    if (SYM) pix[k] = min(i0 + k, n - 1) * n + min(j, n - 1);
+    acc[k] = 0.f;
+  }
+  // centre of the warp's pixels
+  const float wj = (float)(tj0 - K) + 0.5f * (float)(BP_TJ - 1);
+  const float wi = -((float)(i0 - K) + 0.5f * (float)(PPT - 1));
 
-  // full tile (also pixels beyond n, which are computed and discarded) so every thread's
-  // lookup stays inside the staged range
-  const float cj0 = (float)(j0 - R), cj1 = (float)(j0 + BP_TJ - 1 - R);
-  const float ci0 = (float)(i0 - R), ci1 = (float)(i0 + BP_TI - 1 - R);
-  const float fjR = (float)(j - R);
-  float nfiR[BP_PPT];
+  // While chunk c is looked up, the lines of chunk c + 2 are described (one warp, a lane per line) and
+  // those of chunk c + 1 loaded, to be written as pairs at its end: one barrier per chunk.
+  constexpr int PER_WARP = BP_LINES / (BP_THREADS / 32);
+  float held[PER_WARP][3];
+  auto describe = [&](int lc, int ll, int slot) {
+    const int l = lc + ll;
+    if (l >= l1) return;
+    const int d = l / args.n_angles;
+    const int a = l - d * args.n_angles;
+    // full tile (also pixels beyond n, which are computed and discarded) so every thread's lookup
+    // stays inside the staged range: t = (j - K) cos - (i - K) sin at the four corners
+    const float cj0 = (float)(tj0 - K), cj1 = (float)(tj0 + BP_TJ - 1 - K);
+    const float ci0 = (float)(ti0 - K), ci1 = (float)(ti0 + TI - 1 - K);
+    BpLine li;
+    li.cs = args.bp_trig[2 * a];
+    li.sn = args.bp_trig[2 * a + 1];
+    const float t00 = fmaf(cj0, li.cs, -ci0 * li.sn), t01 = fmaf(cj1, li.cs, -ci0 * li.sn);
+    const float t10 = fmaf(cj0, li.cs, -ci1 * li.sn), t11 = fmaf(cj1, li.cs, -ci1 * li.sn);
+    const float tmin = fminf(fminf(t00, t01), fminf(t10, t11));
+    const float tmax = fmaxf(fmaxf(t00, t01), fmaxf(t10, t11));
+    const float t_left = (float)(-K), t_right = (float)(n - 1 - K);
+    li.kind = LINE_FAST;
+    if (tmax < t_left - BP_EDGE_GUARD || tmin > t_right + BP_EDGE_GUARD) {
+      li.kind = LINE_EMPTY;
+    } else if (tmin < t_left + BP_EDGE_GUARD || tmax > t_right - BP_EDGE_GUARD) {
+      li.kind = LINE_CHECKED;
+    }
+    li.kbase = (int)floorf(tmin + (float)K) - 1;
+    li.off = (float)(K - li.kbase);
+    li.w = 1.f;
+    if (SYM && args.weights != nullptr) li.w = args.weights[a * args.n_det + d];
+    if (!SYM && args.line_scale != nullptr) li.w = args.line_scale[a];
+    li.half = 0.5f * (float)(n - 1);
+    li.mid = li.half - (float)li.kbase;
+    sh.line[slot][ll] = li;
+  };
+  // A warp loads and writes lines warp, warp + 8, ... of a chunk.
+  auto load_chunk = [&](int lc, int slot) {
 #pragma unroll
-  for (int k = 0; k < BP_PPT; ++k) nfiR[k] = -(float)(i0 + warp + 8 * k - R);
-
-  float acc[BP_PPT];
+    for (int p = 0; p < PER_WARP; ++p) {
+      const int ll = warp + (BP_THREADS / 32) * p;
+      const bool in = lc + ll < l1 && sh.line[slot][ll].kind != LINE_EMPTY;
+      const int kk = in ? sh.line[slot][ll].kbase + lane : n;
+      const float* line = sino + (int64_t)(lc + ll) * n;
 #pragma unroll
-  for (int k = 0; k < BP_PPT; ++k) acc[k] = 0.f;
-
-  for (int l0 = 0; l0 < n_lines; l0 += BP_LINES) {
-    // ---- stage up to BP_LINES lines: each warp fills 4 lines
-    for (int ll = warp; ll < BP_LINES; ll += BP_THREADS / 32) {
-      const int l = l0 + ll;
-      if (l >= n_lines) break;
-      const int d = l / args.n_angles;
-      const int a = l - d * args.n_angles;
-      const float cs = args.bp_trig[2 * a], sn = args.bp_trig[2 * a + 1];
-      // t = (j - R) cos - (i - R) sin at the four corners
-      const float t00 = fmaf(cj0, cs, -ci0 * sn), t01 = fmaf(cj1, cs, -ci0 * sn);
-      const float t10 = fmaf(cj0, cs, -ci1 * sn), t11 = fmaf(cj1, cs, -ci1 * sn);
-      const float tmin = fminf(fminf(t00, t01), fminf(t10, t11));
-      const float tmax = fmaxf(fmaxf(t00, t01), fmaxf(t10, t11));
-      int kind = LINE_FAST;
-      if (tmax < t_left - BP_EDGE_GUARD || tmin > t_right + BP_EDGE_GUARD) {
-        kind = LINE_EMPTY;
-      } else if (tmin < t_left + BP_EDGE_GUARD || tmax > t_right - BP_EDGE_GUARD) {
-        kind = LINE_CHECKED;
-      }
-      const int kbase = (int)floorf(tmin + (float)K) - 1;
-      float w = 1.f;
-      if (SYM && args.weights != nullptr) w = args.weights[a * args.n_det + d];
-      if (!SYM && args.line_scale != nullptr) w = args.line_scale[a];
-      const float* line = sino + ((int64_t)d * args.n_angles + a) * n;
-      if (kind != LINE_EMPTY) {
-        float v[3], vn[3];
+      for (int q = 0; q < 3; ++q) held[p][q] = (unsigned)(kk + 32 * q) < (unsigned)n ? __ldg(line + kk + 32 * q) : 0.f;
+    }
+  };
+  // (value, slope) pairs, zero outside [0, n - 1)
+  auto store_chunk = [&](int lc, int slot, int buf) {
 #pragma unroll
-        for (int q3 = 0; q3 < 3; ++q3) {
-          const int kk = kbase + lane + 32 * q3;
-          v[q3] = (kk >= 0 && kk < n) ? __ldg(line + kk) : 0.f;
-          vn[q3] = (kk + 1 >= 0 && kk + 1 < n) ? __ldg(line + kk + 1) : 0.f;
-        }
+    for (int p = 0; p < PER_WARP; ++p) {
+      const int ll = warp + (BP_THREADS / 32) * p;
+      if (lc + ll >= l1) break;
+      const int kbase = sh.line[slot][ll].kbase;
+      const float w = sh.line[slot][ll].w;
 #pragma unroll
-        for (int q3 = 0; q3 < 3; ++q3) {
-          const int q = lane + 32 * q3;
-          if (q < BP_KW) pairs[ll][q] = make_float2(w * v[q3], w * (vn[q3] - v[q3]));
-        }
-      }
-      if (lane == 0) {
-        linfo[ll] = make_float4(cs, sn, (float)(K - kbase), w);
-        lkind[ll] = kind;
-        lkbase[ll] = kbase;
-        // the FP32 coordinate u = t + K - kbase of the accumulate loop is within ~1e-4 of its
-        // exact value: pixels with u inside the detector by more than BP_EDGE_GUARD take the
-        // fast lerp, only the others decide the edge in double precision
-        linner[ll] = make_float2((float)(-kbase) + BP_EDGE_GUARD, (float)(n - 1 - kbase) - BP_EDGE_GUARD);
+      for (int q = 0; q < 3; ++q) {
+        float vn = __shfl_down_sync(0xffffffffu, held[p][q], 1);
+        const float v32 = q < 2 ? __shfl_sync(0xffffffffu, held[p][q < 2 ? q + 1 : q], 0) : 0.f;
+        if (lane == 31) vn = v32;
+        const int b = lane + 32 * q;
+        const bool in = (unsigned)(kbase + b) < (unsigned)(n - 1);
+        if (b < BP_KW) sh.pairs[buf][ll][b] = in ? make_float2(w * held[p][q], w * (vn - held[p][q])) : make_float2(0.f, 0.f);
       }
     }
-    __syncthreads();
+  };
 
-    // ---- accumulate
-    const int lines_here = min(BP_LINES, n_lines - l0);
-    for (int ll = 0; ll < lines_here; ++ll) {
-      const int kind = lkind[ll];
+  // (the previous segment's last barrier is behind every thread)
+  if (lane < PER_WARP) describe(l0, warp + (BP_THREADS / 32) * lane, 0);
+  if (warp == BP_THREADS / 32 - 1 && lane < BP_LINES) describe(l0 + BP_LINES, lane, 1);
+  __syncwarp();
+  load_chunk(l0, 0);
+  store_chunk(l0, 0, 0);
+  __syncthreads();
+  int slot = 0, buf = 0;
+  for (int lc = l0, c = 0; lc < l1; lc += BP_LINES, buf ^= 1, ++c) {
+    const int count = min(BP_LINES, l1 - lc);
+    const bool more = lc + BP_LINES < l1;
+    const int next = slot == 2 ? 0 : slot + 1;
+    if (warp == (c & 7) && lane < BP_LINES) describe(lc + 2 * BP_LINES, lane, next == 2 ? 0 : next + 1);
+    if (!SYM && more) load_chunk(lc + BP_LINES, next);  // SYM keeps the registers for its maps
+    const float2 (*pairs)[BP_KW] = sh.pairs[buf];
+    const BpLine* lines = sh.line[slot];
+    unsigned near_edge = 0u;  // lines of the chunk with a pixel of this thread at a detector edge
+    for (int ll = 0; ll < count; ++ll) {
+      const float4 li = *reinterpret_cast<const float4*>(&lines[ll]);
+      const int kind = __float_as_int(li.w);
       if (kind == LINE_EMPTY) continue;
-      const float4 inf = linfo[ll];
-      const float base = fmaf(fjR, inf.x, inf.z);
-      const float2* pr = pairs[ll];
-      int a = 0, d = 0;
+      bool edge = false;
+      if (kind == LINE_CHECKED) {
+        // does a detector edge cross this warp's 32 x PPT pixels?
+        const float uc = fmaf(wi, li.y, fmaf(wj, li.x, li.z));
+        const float reach =
+            fmaf(0.5f * (float)(BP_TJ - 1), fabsf(li.x), 0.5f * (float)(PPT - 1) * fabsf(li.y)) + 2.f * BP_EDGE_GUARD;
+        edge = fabsf(fabsf(uc - lines[ll].mid) - lines[ll].half) < reach;
+      }
+      const float base = fmaf(fj, li.x, li.z);
+      const float2 base2 = make_float2(base, base), sn2 = make_float2(li.y, li.y);
+      // byte offset of the line's bin 0, less the exponent bits of the floors
+      const unsigned row = (unsigned)ll * (unsigned)sizeof(sh.pairs[0][0]) - (0x4B400000u << 3);
+      float m[PPT];
       if (SYM) {
-        const int l = l0 + ll;
-        d = l / args.n_angles;
-        a = l - d * args.n_angles;
-      }
-      if (kind == LINE_FAST && !SYM) {
+        const int l = lc + ll;
+        const int d = l / args.n_angles;
+        const MapRef mr = make_map_ref(args.maps, MAPS_DTYPE, args.maps_slice_stride, args.n_angles, args.n_det, n, s,
+                                       l - d * args.n_angles, d, args.n_channels, args.chan_scale);
 #pragma unroll
-        for (int k = 0; k < BP_PPT; ++k) {
-          const FloorSplit fs = floor_split(fmaf(nfiR[k], inf.y, base));
-          const float2 p = pr[fs.i];
-          acc[k] += fmaf(fs.f, p.y, p.x);
-        }
-        continue;
+        for (int k = 0; k < PPT; ++k) m[k] = map_at<MAPS_DTYPE>(mr, pix[k]);
       }
-      const float2 inner = linner[ll];
+      if (!edge) {
 #pragma unroll
-      for (int k = 0; k < BP_PPT; ++k) {
-        const int i = i0 + warp + 8 * k;
-        const float u = fmaf(nfiR[k], inf.y, base);
-        const FloorSplit fs = floor_split(u);
-        const float2 p = pr[fs.i];
-        float v = fmaf(fs.f, p.y, p.x);
-        if (kind == LINE_CHECKED && !(u > inner.x && u < inner.y)) {
-          // np.interp(t, k - K, line, left=0, right=0) decided in double like numpy
-          const double td = __dsub_rn(__dmul_rn((double)(j - R), (double)inf.x),
-                                      __dmul_rn((double)(i - R), (double)inf.y));
-          if (td < -(double)K || td > (double)(n - 1 - K)) {
-            v = 0.f;
-          } else {
-            const double uk = td + (double)K;
-            const double fl = floor(uk);
-            const int kidx = (int)fl - lkbase[ll];
-            const float2 pe = pr[min(max(kidx, 0), BP_KW - 1)];
-            v = (float)((double)pe.x + (uk - fl) * (double)pe.y);
-          }
+        for (int k = 0; k < PPT; k += 2) {
+          const float2 r = bp_lerp2(pairs, row, __ffma2_rn(nfi[k / 2], sn2, base2));
+          acc[k] = SYM ? acc[k] + r.x * m[k] : acc[k] + r.x;
+          acc[k + 1] = SYM ? acc[k + 1] + r.y * m[k + 1] : acc[k + 1] + r.y;
         }
+      } else {
+        // np.interp's left = right = 0 make the detector edges discontinuous; the FP32 position is
+        // within ~1e-4 of its exact value, so only pixels this close to an edge need more: they are
+        // left out here and added after the chunk
+        const float mid = lines[ll].mid, half = lines[ll].half;
+        bool any = false;
+#pragma unroll
+        for (int k = 0; k < PPT; k += 2) {
+          const float2 u = __ffma2_rn(nfi[k / 2], sn2, base2);
+          float2 r = bp_lerp2(pairs, row, u);
+          const bool e0 = fabsf(fabsf(u.x - mid) - half) < BP_EDGE_GUARD;
+          const bool e1 = fabsf(fabsf(u.y - mid) - half) < BP_EDGE_GUARD;
+          if (e0) r.x = 0.f;
+          if (e1) r.y = 0.f;
+          any = any || e0 || e1;
+          acc[k] = SYM ? acc[k] + r.x * m[k] : acc[k] + r.x;
+          acc[k + 1] = SYM ? acc[k + 1] + r.y * m[k + 1] : acc[k + 1] + r.y;
+        }
+        if (any) near_edge |= 1u << ll;
+      }
+    }
+    for (; near_edge != 0u; near_edge &= near_edge - 1u) {
+      const int ll = __ffs(near_edge) - 1;
+      const BpLine li = lines[ll];
+      const float base = fmaf(fj, li.cs, li.off);
+#pragma unroll
+      for (int k = 0; k < PPT; ++k) {
+        const float u = fmaf(k & 1 ? nfi[k / 2].y : nfi[k / 2].x, li.sn, base);
+        if (fabsf(fabsf(u - li.mid) - li.half) >= BP_EDGE_GUARD) continue;
+        float v = bp_edge_value(pairs[ll] - li.kbase, li.cs, li.sn, n, fj, -(k & 1 ? nfi[k / 2].y : nfi[k / 2].x));
         if (SYM) {
-          if (i < n && j < n) {
-            const MapRef mr = make_map_ref(args.maps, MAPS_DTYPE, args.maps_slice_stride, args.n_angles, args.n_det, n,
-                                           s, a, d, args.n_channels, args.chan_scale);
-            v *= map_at<MAPS_DTYPE>(mr, (int64_t)i * n + j);
-          }
+          const int l = lc + ll;
+          const int d = l / args.n_angles;
+          const MapRef mr = make_map_ref(args.maps, MAPS_DTYPE, args.maps_slice_stride, args.n_angles, args.n_det, n, s,
+                                         l - d * args.n_angles, d, args.n_channels, args.chan_scale);
+          v *= map_at<MAPS_DTYPE>(mr, pix[k]);
         }
         acc[k] += v;
       }
     }
+    if (SYM && more) load_chunk(lc + BP_LINES, next);
+    if (more) store_chunk(lc + BP_LINES, next, buf ^ 1);
+    slot = next;
     __syncthreads();
   }
+}
 
-  if constexpr (EPI == BP_EPI_MLEM || EPI == BP_EPI_SIRT) {
-    bp_epilogue_rows<EPI, BP_PPT>(args, s, i0 + warp, 8, j, acc);
-  } else {
+// One CTA of the back projection: pixel tile `tile` of slice `s`; with CLUSTER, segment `rank` of the
+// cluster's tile, else all segments.
+template <int EPI, bool SYM, int MAPS_DTYPE, int PPT, bool CLUSTER>
+__device__ __forceinline__ void bp_tile(const BpArgs& args, BpShared& sh, int tile, int s, int rank, int ranks) {
+  constexpr int TI = 8 * PPT;
+  const int n = args.n;
+  if (args.active != nullptr && args.active[s] == 0) return;  // every CTA of the cluster
+  const int tiles_j = (n + BP_TJ - 1) / BP_TJ;
+  const int ti = tile / tiles_j;
+  const int ti0 = ti * TI, tj0 = (tile - ti * tiles_j) * BP_TJ;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int j = tj0 + lane;
+  const int i0 = ti0 + PPT * warp;
+  const int n_lines = args.n_det * args.n_angles;
+  const int log2_segs = bp_log2_segments(n_lines), segs = 1 << log2_segs;
+  float acc[PPT];
+  if constexpr (!CLUSTER) {
+    float total[PPT];
+    for (int g = 0; g < segs; ++g) {
+      bp_segment<SYM, MAPS_DTYPE, PPT>(args, sh, s, ti0, tj0, i0, j, (g * n_lines) >> log2_segs,
+                                       ((g + 1) * n_lines) >> log2_segs, acc);
 #pragma unroll
-    for (int k = 0; k < BP_PPT; ++k) {
-      const int i = i0 + warp + 8 * k;
-      if (i < n && j < n) bp_epilogue<EPI>(args, s, i, j, acc[k]);
+      for (int k = 0; k < PPT; ++k) total[k] = g == 0 ? acc[k] : total[k] + acc[k];
     }
+    if constexpr (EPI == BP_EPI_MLEM || EPI == BP_EPI_SIRT) {
+      bp_epilogue_rows<EPI, PPT>(args, s, i0, 1, j, total);
+    } else {
+#pragma unroll
+      for (int k = 0; k < PPT; ++k) {
+        const int i = i0 + k;
+        if (i < n && j < n) bp_epilogue<EPI>(args, s, i, j, total[k]);
+      }
+    }
+  } else {
+    if (rank < segs) {
+      bp_segment<SYM, MAPS_DTYPE, PPT>(args, sh, s, ti0, tj0, i0, j, (rank * n_lines) >> log2_segs,
+                                       ((rank + 1) * n_lines) >> log2_segs, acc);
+    }
+    __syncthreads();
+    float* part = reinterpret_cast<float*>(sh.pairs[0]);  // [TI][32] of this segment
+    if (rank < segs) {
+#pragma unroll
+      for (int k = 0; k < PPT; ++k) part[(i0 - ti0 + k) * BP_TJ + lane] = acc[k];
+    }
+    cluster_sync_all();
+    const int per_rank = TI * BP_TJ / ranks;
+    for (int p = rank * per_rank + tid; p < (rank + 1) * per_rank; p += BP_THREADS) {
+      float v = cluster_load(part + p, 0);
+      for (int g = 1; g < segs; ++g) v += cluster_load(part + p, g);
+      const int pi = ti0 + p / BP_TJ, pj = tj0 + p % BP_TJ;
+      if (pi < n && pj < n) bp_epilogue<EPI>(args, s, pi, pj, v);
+    }
+    cluster_sync_all();  // the others may still read this CTA's sums
+  }
+}
+
+template <int EPI, bool SYM, int MAPS_DTYPE, bool CLUSTER>
+__device__ __forceinline__ void bp_cta(const BpArgs& args, int tile, int s, int rank, int ranks) {
+  __shared__ __align__(16) BpShared sh;
+  if (bp_tile_rows(args.n) == 64) {
+    bp_tile<EPI, SYM, MAPS_DTYPE, 8, CLUSTER>(args, sh, tile, s, rank, ranks);
+  } else {
+    bp_tile<EPI, SYM, MAPS_DTYPE, 4, CLUSTER>(args, sh, tile, s, rank, ranks);
   }
 }
 
 template <int EPI, bool SYM, int MAPS_DTYPE>
 __global__ void __launch_bounds__(BP_THREADS, 4) bp_kernel(BpArgs args) {
-  bp_cta<EPI, SYM, MAPS_DTYPE>(args, blockIdx.x, blockIdx.y);
+  bp_cta<EPI, SYM, MAPS_DTYPE, false>(args, blockIdx.x, blockIdx.y, 0, 1);
 }
 
-// Back projection over groups of slices in one launch: group g's CTAs are (tile, slice),
-// tile fastest.
+// The same over clusters of `ranks` CTAs along x.
 template <int EPI, bool SYM, int MAPS_DTYPE>
-__global__ void __launch_bounds__(BP_THREADS) bp_ragged_kernel(const BpArgs* __restrict__ groups,
-                                                               const int64_t* __restrict__ start, int n_groups) {
-  const int64_t cta = blockIdx.x;
+__global__ void __launch_bounds__(BP_THREADS, 4) bp_cluster_kernel(BpArgs args, int ranks) {
+  const int tile = blockIdx.x / ranks;
+  bp_cta<EPI, SYM, MAPS_DTYPE, true>(args, tile, blockIdx.y, blockIdx.x - tile * ranks, ranks);
+}
+
+// Back projection over groups of slices in one launch: group g's tiles are (tile, slice), tile
+// fastest, each one CTA or one cluster of BP_MAX_RANKS CTAs (CLUSTER).
+constexpr int BP_MAX_RANKS = 8;
+
+template <int EPI, bool SYM, int MAPS_DTYPE, bool CLUSTER>
+__global__ void __launch_bounds__(BP_THREADS, 4) bp_ragged_kernel(const BpArgs* __restrict__ groups,
+                                                                  const int64_t* __restrict__ start, int n_groups) {
+  constexpr int RANKS = CLUSTER ? BP_MAX_RANKS : 1;
+  const int64_t cta = blockIdx.x / RANKS;
   const int g = ragged_group(start, n_groups, cta);
   const BpArgs& a = groups[g];
-  const int tiles = ((a.n + BP_TJ - 1) / BP_TJ) * ((a.n + BP_TI - 1) / BP_TI);
+  const int tiles = bp_tiles(a.n);
   const int64_t local = cta - start[g];
-  bp_cta<EPI, SYM, MAPS_DTYPE>(a, (int)(local % tiles), (int)(local / tiles));
+  bp_cta<EPI, SYM, MAPS_DTYPE, CLUSTER>(a, (int)(local % tiles), (int)(local / tiles), blockIdx.x % RANKS, RANKS);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1214,19 +1409,48 @@ void launch_fp(const FpArgs& a, cudaStream_t st) {
   }
 }
 
+// A kernel over clusters of `ranks` CTAs along x.
+template <typename Kernel, typename... Args>
+static void launch_cluster(Kernel kernel, const dim3& grid, int ranks, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(BP_THREADS);
+  cfg.stream = st;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)ranks;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, kernel, args...);  // a refused launch is the entry point's sticky error
+}
+
+// Tiles of a batch below which the CTAs of a cluster share each tile's lines: the crossing lies between
+// two and three tiles per SM (512^2 x 720: 327 us in clusters, 333 without at 3 slices = 384 tiles, 422
+// and 414 at 4; 256^2 x 360: 144 and 157 at 8 slices = 256 tiles, 203 and 182 at 12).
+constexpr int64_t BP_FEW_TILES = 352;
+
+template <int EPI, bool SYM, int MAPS_DTYPE>
+static void launch_bp_inst(const BpArgs& a, cudaStream_t st) {
+  const int tiles = bp_tiles(a.n), segs = 1 << bp_log2_segments(a.n_det * a.n_angles);
+  if (segs > 1 && (int64_t)tiles * a.n_slices < BP_FEW_TILES) {
+    launch_cluster(bp_cluster_kernel<EPI, SYM, MAPS_DTYPE>, dim3(tiles * segs, a.n_slices), segs, st, a, segs);
+  } else {
+    bp_kernel<EPI, SYM, MAPS_DTYPE><<<dim3(tiles, a.n_slices), BP_THREADS, 0, st>>>(a);
+  }
+}
+
 template <int EPI>
 static void launch_bp_epi(const BpArgs& a, cudaStream_t st) {
-  const int tiles = ((a.n + BP_TJ - 1) / BP_TJ) * ((a.n + BP_TI - 1) / BP_TI);
-  const dim3 grid(tiles, a.n_slices);
-  const bool sym = a.mode == CCT_BP_SYMMETRIC;
-  if (!sym) {
-    bp_kernel<EPI, false, CCT_DTYPE_F32><<<grid, BP_THREADS, 0, st>>>(a);
+  if (a.mode != CCT_BP_SYMMETRIC) {
+    launch_bp_inst<EPI, false, CCT_DTYPE_F32>(a, st);
   } else if (a.maps_dtype == CCT_DTYPE_BF16) {
-    bp_kernel<EPI, true, CCT_DTYPE_BF16><<<grid, BP_THREADS, 0, st>>>(a);
+    launch_bp_inst<EPI, true, CCT_DTYPE_BF16>(a, st);
   } else if (a.maps_dtype == CCT_DTYPE_FIELDS_F32) {
-    bp_kernel<EPI, true, CCT_DTYPE_FIELDS_F32><<<grid, BP_THREADS, 0, st>>>(a);
+    launch_bp_inst<EPI, true, CCT_DTYPE_FIELDS_F32>(a, st);
   } else {
-    bp_kernel<EPI, true, CCT_DTYPE_F32><<<grid, BP_THREADS, 0, st>>>(a);
+    launch_bp_inst<EPI, true, CCT_DTYPE_F32>(a, st);
   }
 }
 
@@ -1254,20 +1478,31 @@ void launch_fp_ragged(const FpArgs* groups, const int64_t* start, int n_groups, 
   }
 }
 
-template <int EPI>
-static void launch_bp_ragged_epi(const BpArgs* g, const int64_t* start, int ng, int64_t ctas, bool sym, int dt,
-                                 cudaStream_t st) {
-  const dim3 grid((unsigned)ctas);
-  if (!sym) {
-    bp_ragged_kernel<EPI, false, CCT_DTYPE_F32><<<grid, BP_THREADS, 0, st>>>(g, start, ng);
-  } else if (dt == CCT_DTYPE_BF16) {
-    bp_ragged_kernel<EPI, true, CCT_DTYPE_BF16><<<grid, BP_THREADS, 0, st>>>(g, start, ng);
-  } else if (dt == CCT_DTYPE_FIELDS_F32) {
-    bp_ragged_kernel<EPI, true, CCT_DTYPE_FIELDS_F32><<<grid, BP_THREADS, 0, st>>>(g, start, ng);
+template <int EPI, bool SYM, int DT>
+static void launch_bp_ragged_inst(const BpArgs* g, const int64_t* start, int ng, int64_t tiles, cudaStream_t st) {
+  if (tiles < BP_FEW_TILES) {
+    launch_cluster(bp_ragged_kernel<EPI, SYM, DT, true>, dim3((unsigned)tiles * BP_MAX_RANKS), BP_MAX_RANKS, st, g, start,
+                   ng);
   } else {
-    bp_ragged_kernel<EPI, true, CCT_DTYPE_F32><<<grid, BP_THREADS, 0, st>>>(g, start, ng);
+    bp_ragged_kernel<EPI, SYM, DT, false><<<(unsigned)tiles, BP_THREADS, 0, st>>>(g, start, ng);
   }
 }
+
+template <int EPI>
+static void launch_bp_ragged_epi(const BpArgs* g, const int64_t* start, int ng, int64_t tiles, bool sym, int dt,
+                                 cudaStream_t st) {
+  if (!sym) {
+    launch_bp_ragged_inst<EPI, false, CCT_DTYPE_F32>(g, start, ng, tiles, st);
+  } else if (dt == CCT_DTYPE_BF16) {
+    launch_bp_ragged_inst<EPI, true, CCT_DTYPE_BF16>(g, start, ng, tiles, st);
+  } else if (dt == CCT_DTYPE_FIELDS_F32) {
+    launch_bp_ragged_inst<EPI, true, CCT_DTYPE_FIELDS_F32>(g, start, ng, tiles, st);
+  } else {
+    launch_bp_ragged_inst<EPI, true, CCT_DTYPE_F32>(g, start, ng, tiles, st);
+  }
+}
+
+int64_t bp_tile_count(int n) { return bp_tiles(n); }
 
 void launch_bp_ragged(const BpArgs* groups, const int64_t* start, int n_groups, int64_t ctas, int epi, bool sym,
                       int maps_dtype, cudaStream_t st) {

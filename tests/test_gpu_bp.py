@@ -1,0 +1,43 @@
+"""GPU: the back projection at the edges of its tiles, line segments and cluster rule, against the
+FP64 oracle: line counts around the segment counts' steps (16, 32, 64 lines) and the chunk of 16,
+sides around the tiles (32, 64) and the tile-height rule (192), angles whose detector edges fall
+exactly on pixels (0, 90 degrees), several detectors, and batches on both sides of the cluster rule
+(equal bits)."""
+
+import numpy as np
+import pytest
+
+from conftest import rel_l2, report
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5  # FP32 sums of at most a few hundred lines against FP64
+
+
+@pytest.mark.parametrize("n,n_ang,n_det", [(2, 4, 1), (3, 15, 1), (31, 16, 1), (32, 17, 1), (33, 31, 1), (64, 32, 1),
+                                           (65, 63, 1), (96, 64, 1), (192, 65, 1), (193, 40, 2), (200, 360, 1)])
+def test_bp_matches_port_and_batches_agree(n, n_ang, n_det):
+    from oracle import port
+    from pycorrectedemissionct_b200 import core
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    dev = torch.device("cuda", 0)
+    angles = np.linspace(0, 2 * np.pi, n_ang, endpoint=False)
+    rng = np.random.default_rng(n + n_ang)
+    # enough slices that the large batch is past the cluster rule for every side
+    s = 352 // max(1, -(-n // 32) * -(-n // (64 if n > 192 else 32))) + 1
+    y = torch.from_numpy(rng.uniform(0.5, 1.5, size=(s, n_det, n_ang, n)).astype(np.float32)).to(dev)
+    maps = torch.from_numpy(rng.uniform(0.3, 1.0, size=(1, n_ang, n_det, n, n)).astype(np.float32)).to(dev)
+    c = core.XrfCore(n, angles, n_det=n_det, device=dev)
+    one = c.bp(y[:1])
+    assert torch.equal(c.bp(y)[:1], one)
+    sym = c.bp(y[:1], "symmetric", maps)
+    assert torch.equal(c.bp(y, "symmetric", maps.expand(s, -1, -1, -1, -1).contiguous())[:1], sym)
+    _, deg32 = port.backend_angles(angles)
+    y64, m64 = y[0].double().cpu().numpy(), maps[0].double().cpu().numpy()
+    e = rel_l2(one[0].cpu().numpy(), port.bp_xrf(y64, m64, deg32))
+    es = rel_l2(sym[0].cpu().numpy(), port.bp_xrf(y64, m64, deg32, is_symmetric=True))
+    report(f"bp n={n} lines={n_ang * n_det}", e, TOL)
+    assert e < TOL and es < TOL

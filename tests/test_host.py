@@ -634,3 +634,35 @@ def test_quarter_turn_quads():
     rad32 = np.array(phantoms.angles(40), dtype=np.float32)
     assert geometry.quarter_turn_quads(rad32, geometry.half_turn_pairs(rad32), np.pi / 3) is None
     assert geometry.quarter_turn_quads(rad32, None, np.pi / 2) is None
+
+
+@pytest.mark.parametrize("n", [2, 3, 33, 64, 251, 512, 8192])
+def test_bp_edge_decision_equals_double(n):
+    """The back projection decides whether a pixel within 0.01 bin of a detector edge is inside from the
+    exact FP32 halves of its two products (bp_edge_value in csrc/cct_project.cu): mirror it and compare
+    with numpy's double decision at every near-edge pixel of many angles, exact edges included."""
+    f, K = np.float32, n // 2
+    rng = np.random.default_rng(n)
+    ang = np.concatenate([np.linspace(0, 2 * np.pi, 72, endpoint=False), rng.uniform(0, 2 * np.pi, 100)]).astype(f)
+    rad = np.deg2rad(np.rad2deg(ang).astype(f))
+    if n <= 64:
+        jj, ii = (v.ravel() for v in np.meshgrid(np.arange(n), np.arange(n)))
+    else:
+        jj, ii = rng.integers(0, n, 20000), rng.integers(0, n, 20000)
+        jj[:300], jj[300:600], ii[600:900], ii[900:1200] = 0, n - 1, 0, n - 1
+    checked = 0
+    for cs, sn in zip(np.cos(rad).astype(f), np.sin(rad).astype(f)):
+        td = (jj - K) * np.float64(cs) - (ii - K) * np.float64(sn)
+        near = np.minimum(abs(td + K), abs(td - (n - 1 - K))) < 0.01
+        td, jc, ic = td[near], (jj[near] - K).astype(f), (ii[near] - K).astype(f)
+        p, q = (jc * cs).astype(f), (-ic * sn).astype(f)
+        pe = (np.float64(jc) * np.float64(cs) - p).astype(f)
+        qe = (np.float64(-ic) * np.float64(sn) - q).astype(f)
+        s = p + q
+        b = s - p
+        se = (p - (s - b)) + (q - b)
+        left = s < f(-0.5)
+        d = (s + np.where(left, f(K), f(-(n - 1 - K)))) + (se + (pe + qe))
+        assert np.array_equal(np.where(left, d >= 0, d <= 0), (td >= -K) & (td <= n - 1 - K))
+        checked += len(td)
+    assert checked > 0

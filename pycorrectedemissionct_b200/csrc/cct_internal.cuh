@@ -1,6 +1,9 @@
 // Internal launch arguments and fused epilogues shared by the projection and solver kernels.
 #pragma once
 
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
 #include "cct_common.cuh"
 
 namespace cct {
@@ -217,5 +220,17 @@ struct ResidualGroup {
 };
 void launch_residual_ragged(const ResidualGroup* groups, const int64_t* slice_start, int n_groups, int64_t slices,
                             cudaStream_t st);
+
+// cuTensorMapEncodeTiled through the runtime's driver entry point (no libcuda link needed)
+inline PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+  static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+                    q == cudaDriverEntryPointSuccess;
+    return ok ? reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p) : nullptr;
+  }();
+  return fn;
+}
 
 }  // namespace cct

@@ -6,17 +6,12 @@
 // Activations are NHWC bfloat16 with channel counts that are multiples of 16.  Weights are
 // [Cout][3][3][Cin] bfloat16 ("K-major": k = tap * Cin + ci).
 //
-// GEMM tile: M = 128 rows (one TMEM lane each), N = BN columns (16..128, FP32 TMEM columns),
-// K blocks of 64 elements staged in shared memory.  Forward (and data-gradient) convolutions use
-// the 128-byte swizzled K-major UMMA layout: 8 lanes gather one tile row's 128 contiguous bytes
-// (four rows per warp load) and write them as 8 chunks XOR-permuted by the row, conflict-free;
-// the weight-gradient GEMM uses the canonical no-swizzle layout (the 16-byte chunk kc of row r
-// at byte kc * ROWS * 16 + r * 16; descriptor start = base + 2s * ROWS * 16, leading-byte offset
-// ROWS * 16, stride-byte offset 128).  Two operand buffers alternate: all 128 threads gather block
-// kb + 1 while the tensor core works on block kb; one elected thread issues the four MMAs of a
-// block and commits them to that buffer's mbarrier.  Every wait is bounded; on timeout the
-// kernel raises g_net_timeout and leaves after waiting once more for its own MMAs.
+// Both GEMMs have M = 128 (one TMEM lane per row) and FP32 accumulators in TMEM, and read their
+// operands as TMA boxes of pixels x channels in the 32-, 64- or 128-byte swizzled layout that the
+// tensor core reads (blocks of 16, 32 or 64 channels).  Every wait is bounded; on timeout the kernel raises
+// g_net_timeout, waits once more for its own copies and leaves.
 
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 
@@ -27,69 +22,104 @@ namespace cct {
 
 __device__ int g_net_timeout = 0;
 
-constexpr int NET_THREADS = 128;
-constexpr int NET_BM = 128;
-constexpr int NET_BK = 64;
+constexpr int NET_TW = 8;                       // tile columns: 8 pixel rows of an operand are one swizzle atom
+constexpr int NET_TH = 16;                      // tile rows of one M = 128 block
 constexpr uint32_t NET_WAIT_LIMIT = 1u << 24;
+constexpr int NET_SMEM_MAX = 223 * 1024;  // dynamic; 4 KB of the 227 are left to the static arrays
 
-enum NetMode : int { NET_FWD = 0, NET_WGRAD = 1 };
+// n / d for n < 2^31 by one multiplication: (n * mul) >> (32 + shift), mul = floor(2^(32 + shift) / d) + 1
+// with 2^shift >= d / 2 (d = 1: mul = 0 stands for n itself).
+struct FastDiv {
+  uint32_t d, mul, shift;
+  FastDiv() = default;
+  explicit FastDiv(int v) : d((uint32_t)v), mul(0), shift(0) {
+    if (v == 1) return;
+    while ((2u << shift) < d) ++shift;
+    mul = (uint32_t)(((1ull << (32 + shift)) / d) + 1);
+  }
+  __device__ __forceinline__ void divmod(int n, int* q, int* r) const {
+    const uint32_t x = mul == 0 ? (uint32_t)n : __umulhi((uint32_t)n, mul) >> shift;
+    *q = (int)x;
+    *r = n - (int)(x * d);
+  }
+};
 
 struct ConvArgs {
   int batch, h, w, cin, cout;
-  int log2_cin;
-  const __nv_bfloat16* x;   // NHWC input (FWD / WGRAD)
-  const __nv_bfloat16* wt;  // [cout][9][cin] (FWD)
-  const __nv_bfloat16* dy;  // NHWC output gradient (WGRAD)
-  const float* bias;        // [cout] or nullptr (FWD)
-  __nv_bfloat16* y;         // NHWC output (FWD)
-  float* dw;                // [cout][9][cin] FP32, accumulated (WGRAD)
-  int relu;                 // FWD epilogue ReLU
-  int64_t m_total, n_total, k_total;  // GEMM sizes
-  int64_t k_split;          // WGRAD: K range per grid.z slice
+  FastDiv by_n, by_x, by_y;  // n_tiles, tiles_x, tiles_y
+  int ck;              // channels per operand block of x (64, 32 or 16: one 128-, 64- or 32-byte swizzled row)
+  int tiles_x, tiles_y, tiles, n_tiles;
+  const float* bias;   // [cout] or nullptr
+  __nv_bfloat16* y;    // NHWC output
+  int relu, wide;      // wide: y is 32-byte aligned
+  int stages, resident;
+};
+
+struct WgradArgs {
+  int batch, h, w, cin, cout;
+  int ckx, cky;        // channels per operand block of x and dy
+  int bx, by;          // operand blocks of x (M) and dy (N) per CTA
+  int n;               // N = by * cky
+  int tiles_x, tiles_y, tiles;
+  int sets;            // MMAs per K step: taps (or groups of taps) of one dx
+  int stages;
+  float* dw;           // [cout][9][cin] FP32, accumulated
 };
 
 __device__ __forceinline__ uint32_t net_smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ uint64_t umma_smem_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr >> 4) & 0x3FFF);
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;  // descriptor version for sm_100
-  // base offset 0, legacy LBO mode, layout type 0 = SWIZZLE_NONE
-  return d;
+// Shared-memory operand of rows of `ck` BF16 elements (128, 64 or 32 bytes) as TMA writes them with the
+// matching swizzle; 8 rows are an atom.  K-major: rows are M / N, lbo unused, sbo = atom.
+// MN-major: rows are K, lbo = distance of the next ck elements along M / N, sbo = atom.
+// The two words of the descriptor: a further operand in the same buffer adds its byte offset / 16 to
+// the low one (one thread issues all MMAs, so what it computes per MMA is what an MMA costs).
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t addr, uint32_t lbo_bytes) {
+  return ((addr >> 4) & 0x3FFF) | (((lbo_bytes >> 4) & 0x3FFF) << 16);
+}
+__device__ __forceinline__ uint32_t umma_desc_hi(int ck) {
+  const uint32_t layout = ck == 64 ? 2 : ck == 32 ? 4 : 6;  // SWIZZLE_128B, _64B, _32B
+  return ((16u * (uint32_t)ck) >> 4)                        // stride-byte offset: 8 rows
+         | (1u << 14)                                       // descriptor version for sm_100
+         | (layout << 29);
+}
+__device__ __forceinline__ uint64_t umma_desc(uint32_t lo, uint32_t hi) { return ((uint64_t)hi << 32) | lo; }
+
+// M = 128, BF16 x BF16 -> FP32; `mn_major`: both operands MN-major
+__device__ __forceinline__ uint32_t umma_idesc(int n, bool mn_major) {
+  return (1u << 4)                            // D format FP32
+         | (1u << 7)                          // A format BF16
+         | (1u << 10)                         // B format BF16
+         | (mn_major ? (3u << 15) : 0u)       // A and B transposed
+         | ((uint32_t)(n >> 3) << 17)         // N / 8
+         | ((uint32_t)(128 >> 4) << 24);      // M / 16
 }
 
-// K-major operand in the 128-byte swizzle layout: row r's 64 K elements (128 bytes) at r * 128 with
-// its 16-byte chunk c stored at chunk c ^ (r % 8), 8-row atoms 1024 bytes apart (stride-byte
-// offset), atom bases 1024-byte aligned; the leading-byte offset (between the two 16-byte chunks
-// of one K = 16 step) is one chunk.  A K = 16 step inside the row advances the start address by
-// 32 bytes; the tensor core applies the swizzle to the address bits.
-__device__ __forceinline__ uint64_t umma_sw128_desc(uint32_t addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr >> 4) & 0x3FFF);
-  d |= (uint64_t)1 << 16;            // leading-byte offset: 16 bytes
-  d |= (uint64_t)(1024 >> 4) << 32;  // stride-byte offset: 1024 bytes
-  d |= (uint64_t)1 << 46;            // descriptor version for sm_100
-  d |= (uint64_t)2 << 61;            // layout type SWIZZLE_128B
-  return d;
+__device__ __forceinline__ void umma_bf16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(acc ? 1u : 0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+      : "memory");
 }
 
-// Byte offset of 16-byte chunk kc of row r in a 128-byte swizzled K-major operand.
-__device__ __forceinline__ uint32_t sw128_offset(int r, int kc) { return (uint32_t)(r * 128 + ((kc ^ (r & 7)) << 4)); }
-
-__host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
-  return (1u << 4)                    // D format FP32
-         | (1u << 7)                  // A format BF16
-         | (1u << 10)                 // B format BF16
-         | ((uint32_t)(n >> 3) << 17) // N / 8
-         | ((uint32_t)(m >> 4) << 24);  // M / 16   (A and B K-major: bits 15, 16 = 0)
+__device__ __forceinline__ void umma_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(net_smem_u32(bar))
+               : "memory");
 }
 
-__device__ __forceinline__ void net_mbar_init(uint64_t* bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(net_smem_u32(bar)) : "memory");
+__device__ __forceinline__ void net_mbar_init(uint64_t* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(net_smem_u32(bar)), "r"(count) : "memory");
 }
-__device__ __forceinline__ bool net_mbar_wait(uint64_t* bar, uint32_t phase) {
+__device__ __forceinline__ void net_mbar_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(net_smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void net_mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(net_smem_u32(bar)) : "memory");
+}
+
+// Bounded wait; when it runs out (or another warp's did) the CTA gives up: abort is set, the flag that
+// the host reads is raised, and every role leaves its loop.
+__device__ __forceinline__ bool net_mbar_wait(uint64_t* bar, uint32_t phase, volatile int* abort) {
   for (uint32_t it = 0; it < NET_WAIT_LIMIT; ++it) {
     uint32_t ok;
     asm volatile(
@@ -98,297 +128,555 @@ __device__ __forceinline__ bool net_mbar_wait(uint64_t* bar, uint32_t phase) {
         : "r"(net_smem_u32(bar)), "r"(phase)
         : "memory");
     if (ok) return true;
+    if (*abort) return false;
   }
+  *abort = 1;
+  atomicExch(&g_net_timeout, 1);
   return false;
 }
 
-__device__ __forceinline__ uint4 zero4() { return make_uint4(0u, 0u, 0u, 0u); }
-
-// 8 consecutive k of the im2col row of output pixel m (k = tap * cin + ci, cin % 8 == 0), with the
-// pixel's coordinates hoisted out of the K loop: px points at input pixel (b, y, x) of output row
-// m (valid = m < m_total).  tap / 3 for tap < 9 is (tap * 11) >> 5.
-__device__ __forceinline__ uint4 load_im2col_row(const ConvArgs& a, const __nv_bfloat16* px, int y, int x, bool valid,
-                                                 int64_t k) {
-  if (!valid || k >= a.k_total) return zero4();
-  const int tap = (int)(k >> a.log2_cin);
-  const int ci = (int)(k & (int64_t)(a.cin - 1));
-  const int ty = (tap * 11) >> 5;
-  const int dy = ty - 1, dx = tap - 3 * ty - 1;
-  const int ys = y + dy, xs = x + dx;
-  if ((unsigned)ys >= (unsigned)a.h || (unsigned)xs >= (unsigned)a.w) return zero4();
-  return __ldg(reinterpret_cast<const uint4*>(px + ((int64_t)dy * a.w + dx) * a.cin + ci));
+__device__ __forceinline__ void tma_4d(void* dst, const CUtensorMap* map, int c, int x, int y, int b, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+      "[%6];" ::"r"(net_smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(c), "r"(x), "r"(y), "r"(b), "r"(net_smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void tma_3d(void* dst, const CUtensorMap* map, int c, int x, int y, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::
+          "r"(net_smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(c), "r"(x), "r"(y), "r"(net_smem_u32(bar))
+      : "memory");
 }
 
-__device__ __forceinline__ uint4 pack8(const __nv_bfloat16 v[8]) {
-  uint4 r;
-  r.x = (uint32_t)__bfloat16_as_ushort(v[0]) | ((uint32_t)__bfloat16_as_ushort(v[1]) << 16);
-  r.y = (uint32_t)__bfloat16_as_ushort(v[2]) | ((uint32_t)__bfloat16_as_ushort(v[3]) << 16);
-  r.z = (uint32_t)__bfloat16_as_ushort(v[4]) | ((uint32_t)__bfloat16_as_ushort(v[5]) << 16);
-  r.w = (uint32_t)__bfloat16_as_ushort(v[6]) | ((uint32_t)__bfloat16_as_ushort(v[7]) << 16);
-  return r;
+__device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(net_smem_u32(slot)), "r"(cols)
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc(uint32_t base, uint32_t cols) {
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols) : "memory");
+}
+__device__ __forceinline__ void tmem_load16(uint32_t addr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
+      "[%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(addr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// WGRAD GEMM: rows m = (tap, ci) (k_total of the forward), columns n = co, k = pixel.
-// A(m, k..k+7) = x[pixel k.. shifted by tap][ci]; B(n, k..k+7) = dy[pixel k..][co].
-__device__ __forceinline__ uint4 load_wgrad_a(const ConvArgs& a, int64_t m, int64_t k) {
-  const int64_t rows = 9LL * a.cin;
-  __nv_bfloat16 v[8];
-  const int tap = (int)(m >> a.log2_cin);
-  const int ci = (int)(m - ((int64_t)tap << a.log2_cin));
-  const int dy_ = tap / 3 - 1, dx_ = tap % 3 - 1;
-  const int hw = a.h * a.w;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    v[j] = __ushort_as_bfloat16((unsigned short)0);
-    const int64_t p = k + j;
-    if (m < rows && p < a.k_total) {
-      const int b = (int)(p / hw);
-      const int rem = (int)(p - (int64_t)b * hw);
-      const int y = rem / a.w, x = rem - (rem / a.w) * a.w;
-      const int ys = y + dy_, xs = x + dx_;
-      if (ys >= 0 && ys < a.h && xs >= 0 && xs < a.w) v[j] = a.x[(((int64_t)b * a.h + ys) * a.w + xs) * a.cin + ci];
-    }
-  }
-  return pack8(v);
+__host__ __device__ inline uint32_t net_tmem_cols(int cols) {
+  uint32_t c = 32;
+  while ((int)c < cols) c *= 2;
+  return c;
 }
 
-__device__ __forceinline__ uint4 load_wgrad_b(const ConvArgs& a, int64_t n, int64_t k) {
-  __nv_bfloat16 v[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    v[j] = __ushort_as_bfloat16((unsigned short)0);
-    const int64_t p = k + j;
-    if (n < a.cout && p < a.k_total) v[j] = a.dy[p * a.cout + n];
-  }
-  return pack8(v);
+// ----------------------------------------------------------------------------------------------
+// Forward (and data-gradient) convolution
+//
+// Persistent CTAs of ten warps: one thread loads operands by TMA, one issues the MMAs, eight warps
+// write the results of the tile before from the other TMEM accumulator (a pair of warps per quarter
+// of its lanes, each with half of the columns: with one warp per quarter and integer divisions
+// for the tile's place, that chain of ~500 dependent instructions was what a tile took).  A tile is 8 columns x 16
+// (or, in pairs that share the weights, 32) rows of output pixels, one TMEM lane each.  For a
+// horizontal tap dx and a block of input channels, one TMA box of 8 x (rows + 2) pixels, zero
+// outside the image, serves the three vertical taps: 8 pixels of a row are one swizzle atom, so a
+// tap is the box from dy rows on.  Weights stay in shared memory for all tiles of a CTA where
+// they fit beside the pixel boxes, and are loaded with each box otherwise.
+// ----------------------------------------------------------------------------------------------
+constexpr int CONV_THREADS = 320;
+
+struct ConvItem {
+  int nt, tx, ty, b;
+};
+__device__ __forceinline__ ConvItem conv_item(const ConvArgs& a, int it) {
+  ConvItem i;
+  int t, u;
+  a.by_n.divmod(it, &t, &i.nt);
+  a.by_x.divmod(t, &u, &i.tx);
+  a.by_y.divmod(u, &i.b, &i.ty);
+  return i;
 }
 
-template <int MODE, int BN>
-__global__ void __launch_bounds__(NET_THREADS) conv_umma_kernel(ConvArgs a) {
-  constexpr int A_BYTES = NET_BM * NET_BK * 2;
-  constexpr int B_BYTES = BN * NET_BK * 2;
-  constexpr int TMEM_COLS = BN < 32 ? 32 : BN;
+template <int MT, int CK>
+__global__ void __launch_bounds__(CONV_THREADS)
+    conv_fwd_kernel(ConvArgs a, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w) {
   extern __shared__ __align__(1024) unsigned char net_smem[];
-  __shared__ __align__(8) uint64_t mma_bar[2];
-  __shared__ uint32_t tmem_base_sh;
-  __shared__ int4 rows_sh[NET_BM];  // FWD: (y, x, output pixel or -1) of every tile row
-
-  unsigned char* abuf[2] = {net_smem, net_smem + A_BYTES};
-  unsigned char* bbuf[2] = {net_smem + 2 * A_BYTES, net_smem + 2 * A_BYTES + B_BYTES};
+  __shared__ __align__(8) uint64_t full[8], empty[8], acc_full[2], acc_empty[2], w_full;
+  __shared__ __align__(16) float bias_sh[512];
+  __shared__ uint32_t tmem_sh;
+  __shared__ int abort_sh;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int64_t m0 = (int64_t)blockIdx.x * NET_BM;
-  const int64_t n0 = (int64_t)blockIdx.y * BN;
-  // forward gather: this thread's output pixel, decomposed once
-  const int64_t m_row = m0 + tid;
-  const bool row_valid = MODE == NET_FWD && m_row < a.m_total;
-  int py = 0, px_ = 0;
-  const __nv_bfloat16* prow = a.x;
-  if (row_valid) {
-    const int hw = a.h * a.w;
-    const int b = (int)(m_row / hw);
-    const int rem = (int)(m_row - (int64_t)b * hw);
-    py = rem / a.w;
-    px_ = rem - py * a.w;
-    prow = a.x + m_row * a.cin;
-  }
-  if (MODE == NET_FWD) rows_sh[tid] = make_int4(py, px_, row_valid ? (int)m_row : -1, 0);
-  int64_t k_begin = 0, k_end = a.k_total;
-  if (MODE == NET_WGRAD) {
-    k_begin = (int64_t)blockIdx.z * a.k_split;
-    k_end = k_begin + a.k_split < a.k_total ? k_begin + a.k_split : a.k_total;
-  }
-  const int kblocks = (int)((k_end - k_begin + NET_BK - 1) / NET_BK);
+  volatile int* abort = &abort_sh;
+  constexpr int ck = CK;
+  const int chunks = a.cin / ck;
+  const int bn = a.cout < 128 ? a.cout : 128;
+  const uint32_t cols = net_tmem_cols(2 * MT * bn);
+  const uint32_t x_bytes = (uint32_t)(NET_TW * (MT * NET_TH + 2) * ck * 2);
+  const uint32_t w_bytes = (uint32_t)(bn * ck * 2);  // one tap
+  const uint32_t x_pitch = (x_bytes + 1023) & ~1023u;
+  const uint32_t stage_bytes = x_pitch + (a.resident ? 0u : 3u * w_bytes);
+  const uint32_t w_base = 0, ring = a.resident ? 9u * chunks * w_bytes : 0u;
+  const int items = a.tiles * a.n_tiles;
 
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(net_smem_u32(&tmem_base_sh)),
-                 "r"(TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == 1) tmem_alloc(&tmem_sh, cols);
+  for (int c = tid; c < a.cout; c += CONV_THREADS) bias_sh[c] = a.bias != nullptr ? a.bias[c] : 0.f;
   if (tid == 0) {
-    net_mbar_init(&mma_bar[0]);
-    net_mbar_init(&mma_bar[1]);
+    for (int s = 0; s < a.stages; ++s) {
+      net_mbar_init(&full[s], 1);
+      net_mbar_init(&empty[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      net_mbar_init(&acc_full[s], 1);
+      net_mbar_init(&acc_empty[s], 8);
+    }
+    net_mbar_init(&w_full, 1);
+    abort_sh = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_d = tmem_base_sh;
-  constexpr uint32_t IDESC = umma_idesc_bf16(NET_BM, BN);
-
-  // A wait that runs out sets this thread's flag; the flags are combined at the block's barrier
-  // (__syncthreads_or), so every thread leaves the loop after the same block.
-  bool timed_out = false;
-  int committed = 0;  // blocks whose MMAs were issued and committed (uniform across the CTA)
-  for (int kb = 0; kb < kblocks; ++kb) {
-    const int buf = kb & 1;
-    if (kb >= 2) {
-      // the MMAs that read this buffer (block kb - 2) must be done before it is overwritten
-      if (!net_mbar_wait(&mma_bar[buf], (uint32_t)(((kb - 2) >> 1) & 1))) timed_out = true;
-    }
-    const int64_t k0 = k_begin + (int64_t)kb * NET_BK;
-    if (MODE == NET_FWD) {
-      // ---- gather A: 8 lanes per tile row, one 16-byte chunk each, so that a warp's load covers
-      // four rows' contiguous K segments; 128-byte swizzled K-major layout
-      uint4 v[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int idx = i * NET_THREADS + tid;
-        const int r = idx >> 3, kc = idx & 7;
-        const int4 ri = rows_sh[r];
-        v[i] = load_im2col_row(a, a.x + (int64_t)max(ri.z, 0) * a.cin, ri.x, ri.y, ri.z >= 0, k0 + 8 * kc);
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int idx = i * NET_THREADS + tid;
-        *reinterpret_cast<uint4*>(abuf[buf] + sw128_offset(idx >> 3, idx & 7)) = v[i];
-      }
-      // ---- gather B: BN weight rows x 8 chunks, same layout
-      for (int it = tid; it < BN * 8; it += NET_THREADS) {
-        const int r = it >> 3, kc = it & 7;
-        const int64_t n = n0 + r;
-        const int64_t k = k0 + 8 * kc;
-        uint4 w = zero4();
-        if (n < a.n_total && k < a.k_total) w = __ldg(reinterpret_cast<const uint4*>(a.wt + n * a.k_total + k));
-        *reinterpret_cast<uint4*>(bbuf[buf] + sw128_offset(r, kc)) = w;
-      }
-    } else {
-      // ---- gather A: 128 rows x 8 chunks (thread = row), canonical no-swizzle layout
-      const int64_t m = m0 + tid;
-#pragma unroll
-      for (int kc = 0; kc < 8; ++kc) {
-        const int64_t k = k0 + 8 * kc;
-        const uint4 v = (k < k_end) ? load_wgrad_a(a, m, k) : zero4();
-        *reinterpret_cast<uint4*>(abuf[buf] + kc * (NET_BM * 16) + tid * 16) = v;
-      }
-      // ---- gather B: BN rows x 8 chunks
-      for (int it = tid; it < BN * 8; it += NET_THREADS) {
-        const int r = it % BN;
-        const int kc = it / BN;
-        const int64_t n = n0 + r;
-        const int64_t k = k0 + 8 * kc;
-        const uint4 v = (k < k_end) ? load_wgrad_b(a, n, k) : zero4();
-        *reinterpret_cast<uint4*>(bbuf[buf] + kc * (BN * 16) + r * 16) = v;
-      }
-    }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (__syncthreads_or(timed_out ? 1 : 0)) {
-      timed_out = true;
-      break;
-    }
-    committed = kb + 1;
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a_base = net_smem_u32(abuf[buf]);
-      const uint32_t b_base = net_smem_u32(bbuf[buf]);
-#pragma unroll
-      for (int s = 0; s < NET_BK / 16; ++s) {
-        const uint64_t ad = MODE == NET_FWD ? umma_sw128_desc(a_base + 32 * s)
-                                            : umma_smem_desc(a_base + 2 * s * NET_BM * 16, NET_BM * 16, 128);
-        const uint64_t bd = MODE == NET_FWD ? umma_sw128_desc(b_base + 32 * s)
-                                            : umma_smem_desc(b_base + 2 * s * BN * 16, BN * 16, 128);
-        const uint32_t acc = (kb > 0 || s > 0) ? 1u : 0u;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem_d),
-            "l"(ad), "l"(bd), "r"(IDESC), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-            : "memory");
-      }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                       net_smem_u32(&mma_bar[buf]))
-                   : "memory");
-    }
   }
-  // wait for the last committed block (its commit covers all earlier MMAs of this thread)
-  if (committed > 0 && !timed_out) {
-    const int last = committed - 1;
-    if (!net_mbar_wait(&mma_bar[last & 1], (uint32_t)((last >> 1) & 1))) timed_out = true;
-  }
-  timed_out = __syncthreads_or(timed_out ? 1 : 0) != 0;
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_sh;
 
-  if (timed_out) {
-    if (tid == 0) {
-      atomicExch(&g_net_timeout, 1);
-      if (committed > 0) {  // one more bounded wait for the MMAs in flight before TMEM is freed
-        const int last = committed - 1;
-        net_mbar_wait(&mma_bar[last & 1], (uint32_t)((last >> 1) & 1));
+  if (warp == 0 && lane == 0) {
+    // ---- loads
+    if (a.resident && blockIdx.x < items) {
+      net_mbar_expect(&w_full, 9u * chunks * w_bytes);
+      for (int c = 0; c < chunks; ++c)
+        for (int t = 0; t < 9; ++t)
+          tma_3d(net_smem + w_base + (uint32_t)(c * 9 + t) * w_bytes, &tm_w, c * ck, t, 0, &w_full);
+    }
+    int s = 0, sent = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
+      const ConvItem i = conv_item(a, it);
+      for (int dx = 0, c = 0; dx < 3; c + 1 == chunks ? (c = 0, ++dx) : ++c) {
+        if (sent >= a.stages && !net_mbar_wait(&empty[s], phase ^ 1u, abort)) {
+          ok = false;
+          break;
+        }
+        unsigned char* st = net_smem + ring + (uint32_t)s * stage_bytes;
+        net_mbar_expect(&full[s], x_bytes + (a.resident ? 0u : 3u * w_bytes));
+        tma_4d(st, &tm_x, c * ck, i.tx * NET_TW + dx - 1, i.ty * MT * NET_TH - 1, i.b, &full[s]);
+        if (!a.resident)
+          for (int dy = 0; dy < 3; ++dy)
+            tma_3d(st + x_pitch + (uint32_t)dy * w_bytes, &tm_w, c * ck, 3 * dy + dx, i.nt * bn, &full[s]);
+        ++sent;
+        if (++s == a.stages) {
+          s = 0;
+          phase ^= 1u;
+        }
       }
     }
-  } else if (kblocks > 0) {
-    // ---- epilogue: warp w owns rows 32w..32w+31 (TMEM lanes), 8 columns per load
-    const int64_t m = m0 + warp * 32 + lane;
-#pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 8) {
-      uint32_t r[8];
-      const uint32_t taddr = tmem_d + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-          : "r"(taddr));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (MODE == NET_FWD) {
-        if (m < a.m_total) {
-          __nv_bfloat16 out[8];
+    if (!ok) {
+      // the copies in flight land before shared memory goes (bounded; abort no longer cuts it short)
+      int none = 0;
+      for (int k = 0; k < a.stages && k < sent; ++k) {
+        const int idx = sent - 1 - k;
+        net_mbar_wait(&full[idx % a.stages], (uint32_t)((idx / a.stages) & 1), &none);
+      }
+    }
+  } else if (warp == 1 && lane == 0) {
+    // ---- MMAs
+    const uint32_t idesc = umma_idesc(bn, false), hi = umma_desc_hi(CK), base = net_smem_u32(net_smem);
+    int s = 0, done = 0, issued = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    if (a.resident && blockIdx.x < items) ok = net_mbar_wait(&w_full, 0, abort);
+    for (int it = blockIdx.x; ok && it < items; it += gridDim.x, ++done) {
+      const int buf = done & 1;
+      if (done >= 2 && !net_mbar_wait(&acc_empty[buf], (uint32_t)(((done >> 1) & 1) ^ 1), abort)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      for (int q = 0, dx = 0, c = 0; q < 3 * chunks; ++q) {
+        if (!net_mbar_wait(&full[s], phase, abort)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t st = base + ring + (uint32_t)s * stage_bytes;
+        const uint32_t xa = umma_desc_lo(st, 16);
+        const uint32_t wb = umma_desc_lo(a.resident ? base + w_base + (uint32_t)(c * 9 + dx) * w_bytes : st + x_pitch, 16);
+        const uint32_t w_step = (a.resident ? 3u * w_bytes : w_bytes) >> 4;
+        const uint32_t acc = tmem + (uint32_t)(buf * MT * bn);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int64_t n = n0 + c0 + j;
-            float v = __uint_as_float(r[j]);
-            if (a.bias != nullptr && n < a.n_total) v += a.bias[n];
-            if (a.relu) v = fmaxf(v, 0.f);
-            out[j] = __float2bfloat16_rn(v);
-          }
-          if (n0 + c0 + 8 <= a.n_total) {
-            *reinterpret_cast<uint4*>(a.y + m * a.n_total + n0 + c0) = pack8(out);
-          } else {
-            for (int j = 0; j < 8; ++j)
-              if (n0 + c0 + j < a.n_total) a.y[m * a.n_total + n0 + c0 + j] = out[j];
+        for (int dy = 0; dy < 3; ++dy) {
+#pragma unroll
+          for (int k = 0; k < CK / 16; ++k) {
+            const uint64_t bd = umma_desc(wb + dy * w_step + 2u * k, hi);
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+              umma_bf16(acc + (uint32_t)(m * bn), umma_desc(xa + (uint32_t)((m * NET_TH + dy) * NET_TW * CK / 8) + 2u * k, hi), bd,
+                        idesc, q > 0 || dy > 0 || k > 0);
           }
         }
-      } else {
-        // dW[co][tap][ci]: row m = (tap, ci), column n = co
-        if (m < 9LL * a.cin) {
+        umma_commit(&empty[s]);
+        ++issued;
+        if (++c == chunks) {
+          c = 0;
+          ++dx;
+        }
+        if (++s == a.stages) {
+          s = 0;
+          phase ^= 1u;
+        }
+      }
+      if (ok) umma_commit(&acc_full[buf]);
+    }
+    if (*abort && issued > 0) {  // the MMAs in flight end before their operands and TMEM go
+      int none = 0;
+      net_mbar_wait(&empty[(issued - 1) % a.stages], (uint32_t)(((issued - 1) / a.stages) & 1), &none);
+    }
+  } else if (warp >= 2) {
+    // ---- results: TMEM lane = pixel, warp % 4 selects its 32 lanes
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    const int row = quarter * 32 + lane;
+    const int c_begin = half * ((bn / 16 + 1) / 2) * 16, c_end = half == 0 ? ((bn / 16 + 1) / 2) * 16 : bn;
+    int done = 0;
+    for (int it = blockIdx.x; it < items; it += gridDim.x, ++done) {
+      const int buf = done & 1;
+      const ConvItem i = conv_item(a, it);
+      const int x = i.tx * NET_TW + (row & 7), n0 = i.nt * bn;
+      const bool ok = net_mbar_wait(&acc_full[buf], (uint32_t)((done >> 1) & 1), abort);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+      for (int m = 0; m < MT; ++m) {
+        const int y = (i.ty * MT + m) * NET_TH + (row >> 3);
+        const bool in = x < a.w && y < a.h;
+        __nv_bfloat16* out = a.y + (((int64_t)i.b * a.h + y) * a.w + x) * a.cout + n0;
+#pragma unroll 1
+        for (int c0 = c_begin; c0 < c_end; c0 += 16) {
+          uint32_t r[16];
+          tmem_load16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((buf * MT + m) * bn + c0), r);
+          if (!in || n0 + c0 >= a.cout) continue;
+          uint32_t o[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int64_t n = n0 + c0 + j;
-            if (n < a.cout) atomicAdd(a.dw + n * (9LL * a.cin) + m, __uint_as_float(r[j]));
+          for (int k = 0; k < 8; ++k) {
+            const float2 bias = *reinterpret_cast<const float2*>(&bias_sh[n0 + c0 + 2 * k]);
+            float v0 = __uint_as_float(r[2 * k]) + bias.x, v1 = __uint_as_float(r[2 * k + 1]) + bias.y;
+            if (a.relu) {
+              v0 = fmaxf(v0, 0.f);
+              v1 = fmaxf(v1, 0.f);
+            }
+            const __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
+            o[k] = *reinterpret_cast<const uint32_t*>(&h);
+          }
+          if (a.wide) {
+            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(out + c0), "r"(o[0]), "r"(o[1]),
+                         "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7])
+                         : "memory");
+          } else {
+            reinterpret_cast<uint4*>(out + c0)[0] = make_uint4(o[0], o[1], o[2], o[3]);
+            reinterpret_cast<uint4*>(out + c0)[1] = make_uint4(o[4], o[5], o[6], o[7]);
           }
         }
       }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) net_mbar_arrive(&acc_empty[buf]);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(TMEM_COLS) : "memory");
-  }
+  if (warp == 1) tmem_dealloc(tmem, cols);
 }
 
-template <int MODE, int BN>
-static int launch_conv_bn(const ConvArgs& a, cudaStream_t st) {
-  // the double-buffered operands; every MMA descriptor addresses inside them (K chunks at
-  // LBO = rows * 16 bytes, core matrices at SBO = 128 bytes), so 3-6 CTAs fit per SM, whose TMEM
-  // columns (BN, at least 32, each) stay within the SM's 512
-  const size_t smem = 2 * (NET_BM * NET_BK * 2) + 2 * (BN * NET_BK * 2);
-  if (!ensure_dynamic_smem<conv_umma_kernel<MODE, BN>>((int)smem)) {
-    cct_set_last_error("cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed for the convolution kernel");
-    return CCT_ERR_CUDA;
+// ----------------------------------------------------------------------------------------------
+// Weight gradient: dW[co][tap][ci] = sum over pixels p of dy[p][co] x[p + tap][ci]
+//
+// A GEMM with M = input channels (of several vertical taps), N = output channels and K = pixels.
+// Both operands are used as TMA brings them (pixels x channels, channels contiguous: MN-major),
+// 128 pixels per stage.  A CTA holds one horizontal tap dx and a range of pixel tiles; its box of
+// x has two more rows, and the next vertical tap is the next atom, so that the descriptor's
+// leading offset of one atom stacks taps along M: four of 32 channels (eight of 16), two of 64,
+// and one of 128 channels (two boxes).  The sums of a tap past the third are not used.
+//
+// 64 x 64 channels over 16 x 128^2 pixels (19 GFLOP, 67 MB): 1465 us with operands gathered element by
+// element, 60 us so.
+//
+// The tensor core's FP32 accumulation truncates, an error that grows with the number of steps (3e-5
+// over 5,000 pixels): every WGRAD_GROUP tiles, 16 steps, the sums go to FP32 registers of eight warps,
+// which add with rounding, while the next group fills the other TMEM buffer.
+// ----------------------------------------------------------------------------------------------
+constexpr int WGRAD_GROUP = 2;
+constexpr int WGRAD_REGS = 8;  // blocks of 16 sums per thread
+
+__global__ void __launch_bounds__(CONV_THREADS)
+    conv_wgrad_kernel(WgradArgs a, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_dy) {
+  extern __shared__ __align__(1024) unsigned char net_smem[];
+  __shared__ __align__(8) uint64_t full[8], empty[8], acc_full[2], acc_empty[2];
+  __shared__ uint32_t tmem_sh;
+  __shared__ int abort_sh;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  volatile int* abort = &abort_sh;
+  const uint32_t cols = net_tmem_cols(2 * a.sets * a.n);
+  const uint32_t x_box = (uint32_t)(NET_TW * (NET_TH + 2) * a.ckx * 2), x_pitch = (x_box + 1023) & ~1023u;
+  const uint32_t dy_box = (uint32_t)(NET_TW * NET_TH * a.cky * 2);
+  const uint32_t stage_bytes = a.bx * x_pitch + a.by * ((dy_box + 1023) & ~1023u);
+  const int dx = blockIdx.y % 3;
+  const int cblock = blockIdx.y / 3;                    // (input block, output block)
+  const int n_blocks = (a.cout + a.n - 1) / a.n;
+  const int ci0 = cblock / n_blocks * a.bx * a.ckx, co0 = cblock % n_blocks * a.n;
+  const int t0 = (int)((int64_t)blockIdx.x * a.tiles / gridDim.x), t1 = (int)((int64_t)(blockIdx.x + 1) * a.tiles / gridDim.x);
+
+  if (warp == 1) tmem_alloc(&tmem_sh, cols);
+  if (tid == 0) {
+    for (int s = 0; s < a.stages; ++s) {
+      net_mbar_init(&full[s], 1);
+      net_mbar_init(&empty[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      net_mbar_init(&acc_full[s], 1);
+      net_mbar_init(&acc_empty[s], 8);
+    }
+    abort_sh = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  dim3 grid((unsigned)((a.m_total + NET_BM - 1) / NET_BM), (unsigned)((a.n_total + BN - 1) / BN), 1);
-  if (MODE == NET_WGRAD) grid.z = (unsigned)((a.k_total + a.k_split - 1) / a.k_split);
-  conv_umma_kernel<MODE, BN><<<grid, NET_THREADS, smem, st>>>(a);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_sh;
+
+  if (warp == 0 && lane == 0) {
+    int s = 0, sent = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = t0; tile < t1; ++tile) {
+      const int tx = tile % a.tiles_x, ty = (tile / a.tiles_x) % a.tiles_y, b = tile / (a.tiles_x * a.tiles_y);
+      if (sent >= a.stages && !net_mbar_wait(&empty[s], phase ^ 1u, abort)) {
+        ok = false;
+        break;
+      }
+      unsigned char* st = net_smem + (uint32_t)s * stage_bytes;
+      net_mbar_expect(&full[s], a.bx * x_box + a.by * dy_box);
+      for (int k = 0; k < a.bx; ++k)
+        tma_4d(st + k * x_pitch, &tm_x, ci0 + k * a.ckx, tx * NET_TW + dx - 1, ty * NET_TH - 1, b, &full[s]);
+      for (int k = 0; k < a.by; ++k)
+        tma_4d(st + a.bx * x_pitch + k * dy_box, &tm_dy, co0 + k * a.cky, tx * NET_TW, ty * NET_TH, b, &full[s]);
+      ++sent;
+      if (++s == a.stages) {
+        s = 0;
+        phase ^= 1u;
+      }
+    }
+    if (!ok) {
+      int none = 0;
+      for (int k = 0; k < a.stages && k < sent; ++k) {
+        const int idx = sent - 1 - k;
+        net_mbar_wait(&full[idx % a.stages], (uint32_t)((idx / a.stages) & 1), &none);
+      }
+    }
+  } else if (warp == 1 && lane == 0) {
+    const uint32_t idesc = umma_idesc(a.n, true);
+    // along M the next ckx rows are the next vertical tap (one atom on), or the next box
+    const uint32_t atom_x = 16u * a.ckx, atom_y = 16u * a.cky;
+    const uint32_t lbo_x = a.bx > 1 ? x_pitch : atom_x, lbo_y = a.by > 1 ? dy_box : atom_y;
+    const uint32_t set_step = ((a.ckx == 64 && a.bx == 1 ? 2u : 1u) * atom_x) >> 4;
+    const uint32_t hi_x = umma_desc_hi(a.ckx), hi_y = umma_desc_hi(a.cky);
+    int s = 0, issued = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = t0; tile < t1; ++tile) {
+      const int group = (tile - t0) / WGRAD_GROUP, in_group = (tile - t0) % WGRAD_GROUP, buf = group & 1;
+      if ((in_group == 0 && group >= 2 && !net_mbar_wait(&acc_empty[buf], (uint32_t)(((group >> 1) & 1) ^ 1), abort)) ||
+          !net_mbar_wait(&full[s], phase, abort)) {
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t d = tmem + (uint32_t)(buf * a.sets * a.n);
+      const uint32_t xs = net_smem_u32(net_smem) + (uint32_t)s * stage_bytes;
+      uint32_t xl = umma_desc_lo(xs, lbo_x), yl = umma_desc_lo(xs + a.bx * x_pitch, lbo_y);
+#pragma unroll
+      for (int k = 0; k < NET_TW * NET_TH / 16; ++k) {  // 16 pixels: two atoms
+        const uint64_t bd = umma_desc(yl, hi_y);
+        const bool acc = in_group > 0 || k > 0;
+        umma_bf16(d, umma_desc(xl, hi_x), bd, idesc, acc);
+        if (a.sets > 1) umma_bf16(d + (uint32_t)a.n, umma_desc(xl + set_step, hi_x), bd, idesc, acc);
+        if (a.sets > 2) umma_bf16(d + (uint32_t)(2 * a.n), umma_desc(xl + 2 * set_step, hi_x), bd, idesc, acc);
+        xl += atom_x >> 3;
+        yl += atom_y >> 3;
+      }
+      umma_commit(&empty[s]);
+      ++issued;
+      if (in_group == WGRAD_GROUP - 1 || tile == t1 - 1) umma_commit(&acc_full[buf]);
+      if (++s == a.stages) {
+        s = 0;
+        phase ^= 1u;
+      }
+    }
+    if (!ok && issued > 0) {
+      int none = 0;
+      net_mbar_wait(&empty[(issued - 1) % a.stages], (uint32_t)(((issued - 1) / a.stages) & 1), &none);
+    }
+  } else if (warp >= 2) {
+    // a pair of warps per quarter of the lanes, each with every other block of 16 columns
+    const int quarter = warp & 3, half = (warp - 2) >> 2, row = quarter * 32 + lane;
+    const int blocks = a.sets * a.n / 16;
+    float sum[WGRAD_REGS][16];
+#pragma unroll
+    for (int j = 0; j < WGRAD_REGS; ++j)
+#pragma unroll
+      for (int k = 0; k < 16; ++k) sum[j][k] = 0.f;
+    const int groups = (t1 - t0 + WGRAD_GROUP - 1) / WGRAD_GROUP;
+    bool ok = true;
+    for (int g = 0; g < groups; ++g) {
+      const int buf = g & 1;
+      ok = __all_sync(0xffffffffu, net_mbar_wait(&acc_full[buf], (uint32_t)((g >> 1) & 1), abort)) != 0;
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int j = 0; j < WGRAD_REGS; ++j) {
+        if (2 * j + half < blocks) {
+          uint32_t r[16];
+          tmem_load16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * a.sets * a.n + (2 * j + half) * 16), r);
+#pragma unroll
+          for (int k = 0; k < 16; ++k) sum[j][k] += __uint_as_float(r[k]);
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) net_mbar_arrive(&acc_empty[buf]);
+    }
+    if (ok) {
+#pragma unroll
+      for (int j = 0; j < WGRAD_REGS; ++j) {
+        const int col = (2 * j + half) * 16, m = col / a.n, c0 = col - m * a.n;
+        const int in_set = a.bx > 1 ? 0 : row / a.ckx;
+        const int dy = m * (a.ckx == 64 && a.bx == 1 ? 2 : 1) + in_set;
+        const int ci = ci0 + (a.bx > 1 ? row : row - in_set * a.ckx);
+        if (2 * j + half >= blocks || dy >= 3 || ci >= a.cin) continue;
+        float* out = a.dw + (3 * dy + dx) * a.cin + ci;
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+          if (co0 + c0 + k < a.cout) atomicAdd(out + (int64_t)(co0 + c0 + k) * 9 * a.cin, sum[j][k]);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem, cols);
+}
+
+// ----------------------------------------------------------------------------------------------
+// Launchers
+// ----------------------------------------------------------------------------------------------
+static int net_sms() {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+static CUtensorMapSwizzle net_swizzle(int ck) {
+  return ck == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : ck == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
+}
+
+// NHWC activations as (channel, x, y, image) with a box of ck channels x 8 columns x `rows` rows.
+static bool net_map_nhwc(CUtensorMap* map, const void* p, int b, int h, int w, int c, int ck, int rows) {
+  PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
+  if (enc == nullptr) return false;
+  const cuuint64_t dims[4] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)b};
+  const cuuint64_t strides[3] = {(cuuint64_t)c * 2, (cuuint64_t)c * 2 * w, (cuuint64_t)c * 2 * w * h};
+  const cuuint32_t box[4] = {(cuuint32_t)ck, (cuuint32_t)NET_TW, (cuuint32_t)rows, 1};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(p), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, net_swizzle(ck), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Weights [cout][9][cin] as (channel, tap, output channel) with a box of one tap of bn outputs.
+static bool net_map_weights(CUtensorMap* map, const void* p, int cin, int cout, int ck, int bn) {
+  PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
+  if (enc == nullptr) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)cin, 9, (cuuint64_t)cout};
+  const cuuint64_t strides[2] = {(cuuint64_t)cin * 2, (cuuint64_t)cin * 18};
+  const cuuint32_t box[3] = {(cuuint32_t)ck, 1, (cuuint32_t)bn};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(p), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, net_swizzle(ck), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+static int net_fail(const char* msg) {
+  cct_set_last_error(msg);
+  return CCT_ERR_CUDA;
+}
+
+template <int MT, int CK>
+static int launch_conv_fwd(ConvArgs a, const void* x, const void* wt, cudaStream_t st) {
+  const int bn = a.cout < 128 ? a.cout : 128, chunks = a.cin / a.ck;
+  a.tiles_x = (a.w + NET_TW - 1) / NET_TW;
+  a.tiles_y = (a.h + MT * NET_TH - 1) / (MT * NET_TH);
+  a.n_tiles = (a.cout + bn - 1) / bn;
+  const int64_t tiles = (int64_t)a.batch * a.tiles_x * a.tiles_y;
+  if (tiles * a.n_tiles > 0x7fffffffLL) return net_fail("the convolution has too many tiles");
+  a.tiles = (int)tiles;
+  a.by_n = FastDiv(a.n_tiles);
+  a.by_x = FastDiv(a.tiles_x);
+  a.by_y = FastDiv(a.tiles_y);
+  const int x_pitch = (NET_TW * (MT * NET_TH + 2) * a.ck * 2 + 1023) / 1024 * 1024, w_tap = bn * a.ck * 2;
+  const int weights = 9 * chunks * w_tap;
+  const int stage = x_pitch + (a.resident ? 0 : 3 * w_tap);
+  const int fixed = a.resident ? weights : 0;
+  // two CTAs per SM where each still gets three stages, else as many stages as one CTA can hold
+  const int half = 110 * 1024;
+  const int per_sm = fixed + 3 * stage <= half && 2 * net_tmem_cols(2 * MT * bn) <= 512 ? 2 : 1;
+  const int room = (per_sm == 2 ? half : NET_SMEM_MAX - 1024) - fixed;
+  a.stages = std::min(8, room / stage);
+  if (a.stages < 2) return net_fail("the convolution's operands do not fit in shared memory");
+  const int smem = fixed + a.stages * stage + 1024;
+  CUtensorMap tm_x, tm_w;
+  if (!net_map_nhwc(&tm_x, x, a.batch, a.h, a.w, a.cin, a.ck, MT * NET_TH + 2) ||
+      !net_map_weights(&tm_w, wt, a.cin, a.cout, a.ck, bn))
+    return net_fail("cuTensorMapEncodeTiled refused the convolution's operands");
+  if (!ensure_dynamic_smem<conv_fwd_kernel<MT, CK>>(NET_SMEM_MAX))
+    return net_fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed for the convolution kernel");
+  const int64_t grid = std::min<int64_t>(tiles * a.n_tiles, (int64_t)net_sms() * per_sm);
+  conv_fwd_kernel<MT, CK><<<(unsigned)grid, CONV_THREADS, smem, st>>>(a, tm_x, tm_w);
   return CCT_OK;
 }
 
-template <int MODE>
-static int launch_conv_mode(const ConvArgs& a, int bn, cudaStream_t st) {
-  switch (bn) {
-    case 16: return launch_conv_bn<MODE, 16>(a, st);
-    case 32: return launch_conv_bn<MODE, 32>(a, st);
-    case 64: return launch_conv_bn<MODE, 64>(a, st);
-    default: return launch_conv_bn<MODE, 128>(a, st);
-  }
+static int net_block(int c) { return c % 64 == 0 ? 64 : c % 32 == 0 ? 32 : 16; }
+
+static int launch_conv_wgrad(WgradArgs a, const void* x, const void* dy, cudaStream_t st) {
+  a.ckx = net_block(a.cin);
+  a.cky = net_block(a.cout);
+  a.bx = a.cin >= 128 ? 2 : 1;                               // cin is a power of two
+  a.sets = a.bx > 1 ? 3 : a.ckx == 64 ? 2 : 1;
+  // two buffers of sets x N sums fit the 512 TMEM columns and the registers of the eight warps
+  a.by = std::max(1, std::min(a.cout, a.sets == 3 ? 64 : 128) / a.cky);
+  a.n = a.by * a.cky;
+  a.tiles_x = (a.w + NET_TW - 1) / NET_TW;
+  a.tiles_y = (a.h + NET_TH - 1) / NET_TH;
+  const int64_t tiles = (int64_t)a.batch * a.tiles_x * a.tiles_y;
+  if (tiles > 0x7fffffffLL) return net_fail("the convolution has too many tiles");
+  a.tiles = (int)tiles;
+  const int x_pitch = (NET_TW * (NET_TH + 2) * a.ckx * 2 + 1023) / 1024 * 1024;
+  const int dy_pitch = (NET_TW * NET_TH * a.cky * 2 + 1023) / 1024 * 1024;
+  const int stage = a.bx * x_pitch + a.by * dy_pitch;
+  a.stages = std::min(8, (NET_SMEM_MAX - 2048) / stage);
+  // the taps past the third read up to five rows past the last box: 2048 spare bytes behind it
+  const int smem = a.stages * stage + 2048;
+  CUtensorMap tm_x, tm_dy;
+  if (!net_map_nhwc(&tm_x, x, a.batch, a.h, a.w, a.cin, a.ckx, NET_TH + 2) ||
+      !net_map_nhwc(&tm_dy, dy, a.batch, a.h, a.w, a.cout, a.cky, NET_TH))
+    return net_fail("cuTensorMapEncodeTiled refused the convolution's operands");
+  if (!ensure_dynamic_smem<conv_wgrad_kernel>(NET_SMEM_MAX))
+    return net_fail("cudaFuncSetAttribute(MaxDynamicSharedMemorySize) failed for the weight-gradient kernel");
+  const int groups = 3 * (a.cin / (a.bx * a.ckx)) * ((a.cout + a.n - 1) / a.n);
+  // one CTA per SM over all groups, at least four tiles each (every CTA adds its sums atomically)
+  const int split = (int)std::max<int64_t>(1, std::min<int64_t>(net_sms() / groups, (tiles + 3) / 4));
+  conv_wgrad_kernel<<<dim3(split, groups), CONV_THREADS, smem, st>>>(a, tm_x, tm_dy);
+  return CCT_OK;
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -401,64 +689,146 @@ __global__ void relu_bwd_kernel(const __nv_bfloat16* y, const __nv_bfloat16* dy,
   }
 }
 
-// 2x2 average pooling (stride 2) and its adjoint
-__global__ void avgpool2_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, int b, int h, int w, int c, int bwd) {
-  const int ho = h / 2, wo = w / 2;
-  const int64_t n = (int64_t)b * ho * wo * c;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int ch = (int)(i % c);
-    int64_t p = i / c;
-    const int xo = (int)(p % wo); p /= wo;
-    const int yo = (int)(p % ho);
-    const int bb = (int)(p / ho);
-    const int64_t base = (((int64_t)bb * h + 2 * yo) * w + 2 * xo) * c + ch;
-    if (!bwd) {
-      const float s = __bfloat162float(x[base]) + __bfloat162float(x[base + c]) +
-                      __bfloat162float(x[base + (int64_t)w * c]) + __bfloat162float(x[base + (int64_t)w * c + c]);
-      y[i] = __float2bfloat16_rn(0.25f * s);
-    } else {
-      // x: gradient at the pooled resolution (index i), y: gradient at full resolution
-      const __nv_bfloat16 g = __float2bfloat16_rn(0.25f * __bfloat162float(x[i]));
-      y[base] = g; y[base + c] = g; y[base + (int64_t)w * c] = g; y[base + (int64_t)w * c + c] = g;
+// Eight BF16 channels (16 bytes) at a time: the tensors' channel counts are multiples of 16.
+struct Bf16x8 {
+  uint4 v;
+  __device__ __forceinline__ void get(float (&f)[8]) const {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      f[2 * k] = __uint_as_float(w[k] << 16);
+      f[2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
+    }
+  }
+  __device__ __forceinline__ void set(const float (&f)[8]) {
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
+      w[k] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    v = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+};
+
+// 2x2 average pooling (stride 2) and its adjoint, V channels per thread (8, or 1 for channel counts or
+// addresses that do not allow 16-byte accesses); grid y: rows of the small images.
+// (Element by element with four divisions each, the network's three pools took 177 us on 8 x 512^2,
+// the upsamplings 288 us and the additions 277 us, 4-5 times their memory time.)
+template <int V>
+__device__ __forceinline__ void ew_load(const __nv_bfloat16* p, float (&f)[V]) {
+  if constexpr (V == 8) {
+    Bf16x8 t;
+    t.v = __ldg(reinterpret_cast<const uint4*>(p));
+    t.get(f);
+  } else {
+    f[0] = __bfloat162float(*p);
+  }
+}
+template <int V>
+__device__ __forceinline__ void ew_store(__nv_bfloat16* p, const float (&f)[V]) {
+  if constexpr (V == 8) {
+    Bf16x8 t;
+    t.set(f);
+    *reinterpret_cast<uint4*>(p) = t.v;
+  } else {
+    *p = __float2bfloat16_rn(f[0]);
+  }
+}
+
+// One row pair of the large image (row pitch `row` elements) and one row of the small one; `half`: the
+// small image is their 2x2 mean (else their sum).  TO_SMALL reduces, else the small value (times 1/4
+// for `half`) goes to the four large pixels.
+template <int V, bool TO_SMALL>
+__global__ void __launch_bounds__(256) resize2_kernel(const __nv_bfloat16* src, __nv_bfloat16* dst, int64_t rows, int w,
+                                                      int c, int half) {
+  // rows (of all images) and w: the small images
+  const int cv = c / V, per_row = w * cv;
+  for (int64_t y = blockIdx.y; y < rows; y += gridDim.y) {
+    const __nv_bfloat16* s = src + y * (TO_SMALL ? 4 : 1) * (int64_t)w * c;
+    __nv_bfloat16* d = dst + y * (TO_SMALL ? 1 : 4) * (int64_t)w * c;
+    const int64_t row = 2 * (int64_t)w * c;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < per_row; i += gridDim.x * blockDim.x) {
+      const int x = i / cv, ch = (i - x * cv) * V;
+      const int64_t big = 2 * (int64_t)x * c + ch, small = (int64_t)x * c + ch;
+      float v[V];
+      if constexpr (TO_SMALL) {
+        float a[V], b[V], e[V], f[V];
+        ew_load<V>(s + big, a);
+        ew_load<V>(s + big + c, b);
+        ew_load<V>(s + big + row, e);
+        ew_load<V>(s + big + row + c, f);
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+          const float t = a[k] + b[k] + e[k] + f[k];
+          v[k] = half ? 0.25f * t : t;
+        }
+        ew_store<V>(d + small, v);
+      } else {
+        ew_load<V>(s + small, v);
+#pragma unroll
+        for (int k = 0; k < V; ++k) v[k] = half ? 0.25f * v[k] : v[k];
+        ew_store<V>(d + big, v);
+        ew_store<V>(d + big + c, v);
+        ew_store<V>(d + big + row, v);
+        ew_store<V>(d + big + row + c, v);
+      }
     }
   }
 }
 
-// nearest 2x upsampling and its adjoint (sum of the 4 children)
-__global__ void upsample2_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, int b, int h, int w, int c, int bwd) {
-  // h, w: the small resolution
-  const int64_t n = (int64_t)b * h * w * c;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int ch = (int)(i % c);
-    int64_t p = i / c;
-    const int xs = (int)(p % w); p /= w;
-    const int ys = (int)(p % h);
-    const int bb = (int)(p / h);
-    const int64_t base = (((int64_t)bb * 2 * h + 2 * ys) * 2 * w + 2 * xs) * c + ch;
-    const int64_t row = (int64_t)2 * w * c;
-    if (!bwd) {
-      const __nv_bfloat16 v = x[i];
-      y[base] = v; y[base + c] = v; y[base + row] = v; y[base + row + c] = v;
-    } else {
-      const float s = __bfloat162float(x[base]) + __bfloat162float(x[base + c]) + __bfloat162float(x[base + row]) +
-                      __bfloat162float(x[base + row + c]);
-      y[i] = __float2bfloat16_rn(s);
-    }
+template <int V>
+__global__ void __launch_bounds__(256) add_kernel(const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat16* out,
+                                                  int64_t n) {
+  for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * V; i < n; i += (int64_t)gridDim.x * blockDim.x * V) {
+    float u[V], v[V];
+    ew_load<V>(a + i, u);
+    ew_load<V>(b + i, v);
+#pragma unroll
+    for (int k = 0; k < V; ++k) u[k] += v[k];
+    ew_store<V>(out + i, u);
   }
 }
 
-__global__ void add_kernel(const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat16* out, int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = __float2bfloat16_rn(__bfloat162float(a[i]) + __bfloat162float(b[i]));
-}
-
-// db[c] += sum over pixels of dy[p][c]
-__global__ void bias_grad_kernel(const __nv_bfloat16* dy, float* db, int64_t pixels, int c) {
-  const int ch = blockIdx.y * blockDim.x + threadIdx.x;
-  if (ch >= c) return;
-  float s = 0.f;
-  for (int64_t p = blockIdx.x; p < pixels; p += gridDim.x) s += __bfloat162float(dy[p * c + ch]);
-  atomicAdd(db + ch, s);
+// db[c] += sum over pixels of dy[p][c]: V channels per thread, the threads of a block over pixels,
+// combined in shared memory before one atomic per channel and block.
+template <int V>
+__global__ void __launch_bounds__(256) bias_grad_kernel(const __nv_bfloat16* dy, float* db, int64_t pixels, int c) {
+  __shared__ float part[256 * V];
+  const int cv = min(c / V, 256);              // channel groups of this block (blockIdx.y: the next 256)
+  const int lanes = 256 / cv, g = threadIdx.x % cv, lane = threadIdx.x / cv;
+  const int ch = (blockIdx.y * 256 + g) * V;
+  float s[V];
+#pragma unroll
+  for (int k = 0; k < V; ++k) s[k] = 0.f;
+  if (lane < lanes && ch < c) {
+    const int64_t step = (int64_t)gridDim.x * lanes;
+    int64_t p = (int64_t)blockIdx.x * lanes + lane;
+    for (; p + 7 * step < pixels; p += 8 * step) {  // eight loads in flight
+      float v[8][V];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) ew_load<V>(dy + (p + u * step) * c + ch, v[u]);
+#pragma unroll
+      for (int k = 0; k < V; ++k)
+        s[k] += ((v[0][k] + v[1][k]) + (v[2][k] + v[3][k])) + ((v[4][k] + v[5][k]) + (v[6][k] + v[7][k]));
+    }
+    for (; p < pixels; p += step) {
+      float v[V];
+      ew_load<V>(dy + p * c + ch, v);
+#pragma unroll
+      for (int k = 0; k < V; ++k) s[k] += v[k];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < V; ++k) part[threadIdx.x * V + k] = s[k];
+  __syncthreads();
+  if (lane == 0 && ch < c) {
+    for (int l = 1; l < lanes; ++l)
+#pragma unroll
+      for (int k = 0; k < V; ++k) s[k] += part[(l * cv + g) * V + k];
+#pragma unroll
+    for (int k = 0; k < V; ++k) atomicAdd(db + ch + k, s[k]);
+  }
 }
 
 // MSE loss on channel 0 of an NHWC prediction vs an FP32 target [b][h][w]:
@@ -548,6 +918,46 @@ static inline unsigned ew_blocks(int64_t n) {
   return (unsigned)(b < 1 ? 1 : b);
 }
 
+// 16-byte accesses: every address and the channel count allow them
+static bool ew_wide(const void* a, const void* b, const void* d, int64_t c) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(d)) & 15) == 0 &&
+         c % 8 == 0;
+}
+
+// small (h x w) and large (2h x 2w) images of c channels
+static void launch_resize2(const void* src, void* dst, int64_t rows, int w, int c, int half, bool to_small,
+                           cudaStream_t st) {
+  const bool wide = ew_wide(src, dst, nullptr, c);
+  const int per_row = w * (wide ? c / 8 : c);
+  const dim3 grid((unsigned)std::min(64, (per_row + 255) / 256), (unsigned)std::min<int64_t>(rows, 65535));
+  const __nv_bfloat16* s = reinterpret_cast<const __nv_bfloat16*>(src);
+  __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(dst);
+  if (wide && to_small) {
+    resize2_kernel<8, true><<<grid, 256, 0, st>>>(s, d, rows, w, c, half);
+  } else if (wide) {
+    resize2_kernel<8, false><<<grid, 256, 0, st>>>(s, d, rows, w, c, half);
+  } else if (to_small) {
+    resize2_kernel<1, true><<<grid, 256, 0, st>>>(s, d, rows, w, c, half);
+  } else {
+    resize2_kernel<1, false><<<grid, 256, 0, st>>>(s, d, rows, w, c, half);
+  }
+}
+
+static void launch_bias_grad(const void* dy, float* db, int64_t pixels, int c, cudaStream_t st) {
+  const __nv_bfloat16* p = reinterpret_cast<const __nv_bfloat16*>(dy);
+  const bool wide = ew_wide(dy, nullptr, nullptr, c);
+  const int groups = wide ? c / 8 : c, lanes = 256 / std::min(groups, 256);
+  // 16 pixels per thread, or more where that takes over two blocks per SM (every block adds its sums
+  // to the same few addresses: 512 blocks of 64 channels took 25 us on 33 MB)
+  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(2 * net_sms(), pixels / (16 * lanes)));
+  const dim3 grid((unsigned)blocks, (unsigned)((groups + 255) / 256));
+  if (wide) {
+    bias_grad_kernel<8><<<grid, 256, 0, st>>>(p, db, pixels, c);
+  } else {
+    bias_grad_kernel<1><<<grid, 256, 0, st>>>(p, db, pixels, c);
+  }
+}
+
 int read_net_timeout(int clear, int* value) {
   int v = 0;
   cudaError_t e = cudaMemcpyFromSymbol(&v, g_net_timeout, sizeof(int));
@@ -574,20 +984,8 @@ static int net_check_conv(const cct_conv_desc* d) {
   return CCT_OK;
 }
 
-static cct::ConvArgs net_args(const cct_conv_desc* d) {
-  cct::ConvArgs a;
-  std::memset(&a, 0, sizeof(a));
-  a.batch = d->batch; a.h = d->height; a.w = d->width; a.cin = d->cin; a.cout = d->cout;
-  int l = 0;
-  while ((1 << l) < d->cin) ++l;
-  a.log2_cin = l;
-  return a;
-}
-
-// the implicit-GEMM loads move 8 bf16 (16 bytes) at a time
+// TMA reads tensors that start on 16-byte boundaries
 static bool net_aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-
-static int net_bn(int cout) { return cout >= 128 ? 128 : cout; }
 
 static int net_launch_check() {
   const cudaError_t e = cudaGetLastError();
@@ -606,16 +1004,27 @@ int cct_conv3x3_fwd(const cct_conv_desc* desc, const void* x, const void* w, con
   if (rc != CCT_OK) return rc;
   CCT_REQUIRE(x != nullptr && w != nullptr && y != nullptr, "x, w and y are required");
   CCT_REQUIRE(net_aligned16(x) && net_aligned16(w) && net_aligned16(y), "x, w and y must be 16-byte aligned");
-  cct::ConvArgs a = net_args(desc);
-  a.x = reinterpret_cast<const __nv_bfloat16*>(x);
-  a.wt = reinterpret_cast<const __nv_bfloat16*>(w);
+  cct::ConvArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.batch = desc->batch; a.h = desc->height; a.w = desc->width; a.cin = desc->cin; a.cout = desc->cout;
+  a.ck = desc->cin < 64 ? desc->cin : 64;
   a.bias = bias;
   a.y = reinterpret_cast<__nv_bfloat16*>(y);
   a.relu = relu;
-  a.m_total = (int64_t)desc->batch * desc->height * desc->width;
-  a.n_total = desc->cout;
-  a.k_total = 9LL * desc->cin;
-  rc = cct::launch_conv_mode<cct::NET_FWD>(a, net_bn(desc->cout), reinterpret_cast<cudaStream_t>(stream));
+  a.wide = (reinterpret_cast<uintptr_t>(y) & 31) == 0;
+  // weights of one output tile stay in shared memory up to 74 KB (64 x 64 channels); beyond that two
+  // pixel tiles share each load of them
+  a.resident = desc->cout <= 128 && 9 * desc->cin * desc->cout * 2 <= 9 * 64 * 64 * 2;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (a.resident) {
+    rc = a.ck == 64   ? cct::launch_conv_fwd<1, 64>(a, x, w, st)
+         : a.ck == 32 ? cct::launch_conv_fwd<1, 32>(a, x, w, st)
+                      : cct::launch_conv_fwd<1, 16>(a, x, w, st);
+  } else {
+    rc = a.ck == 64   ? cct::launch_conv_fwd<2, 64>(a, x, w, st)
+         : a.ck == 32 ? cct::launch_conv_fwd<2, 32>(a, x, w, st)
+                      : cct::launch_conv_fwd<2, 16>(a, x, w, st);
+  }
   if (rc != CCT_OK) return rc;
   return net_launch_check();
 }
@@ -625,21 +1034,11 @@ int cct_conv3x3_wgrad(const cct_conv_desc* desc, const void* x, const void* dy, 
   if (rc != CCT_OK) return rc;
   CCT_REQUIRE(x != nullptr && dy != nullptr && dw != nullptr, "x, dy and dw are required");
   CCT_REQUIRE(net_aligned16(x) && net_aligned16(dy), "x and dy must be 16-byte aligned");
-  cct::ConvArgs a = net_args(desc);
-  a.x = reinterpret_cast<const __nv_bfloat16*>(x);
-  a.dy = reinterpret_cast<const __nv_bfloat16*>(dy);
+  cct::WgradArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.batch = desc->batch; a.h = desc->height; a.w = desc->width; a.cin = desc->cin; a.cout = desc->cout;
   a.dw = dw;
-  a.m_total = 9LL * desc->cin;
-  a.n_total = desc->cout;
-  a.k_total = (int64_t)desc->batch * desc->height * desc->width;
-  // split K (pixels) so that the grid has a few hundred CTAs
-  const int64_t tiles = ((a.m_total + 127) / 128) * ((a.n_total + 127) / 128);
-  int64_t splits = (512 + tiles - 1) / tiles;
-  int64_t ks = (a.k_total + splits - 1) / splits;
-  ks = ((ks + 63) / 64) * 64;
-  if (ks < 64) ks = 64;
-  a.k_split = ks;
-  rc = cct::launch_conv_mode<cct::NET_WGRAD>(a, net_bn(desc->cout), reinterpret_cast<cudaStream_t>(stream));
+  rc = cct::launch_conv_wgrad(a, x, dy, reinterpret_cast<cudaStream_t>(stream));
   if (rc != CCT_OK) return rc;
   return net_launch_check();
 }
@@ -663,36 +1062,35 @@ int cct_net_relu_bwd(const void* y, const void* dy, void* dx, int64_t count, voi
 int cct_net_avgpool2(const void* x, void* y, int32_t batch, int32_t height, int32_t width, int32_t channels,
                      int32_t backward, void* stream) {
   CCT_REQUIRE(x && y && batch > 0 && height % 2 == 0 && width % 2 == 0 && channels > 0, "bad avgpool2 arguments");
-  const int64_t n = (int64_t)batch * (height / 2) * (width / 2) * channels;
-  cct::avgpool2_kernel<<<cct::ew_blocks(n), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<__nv_bfloat16*>(y), batch, height, width, channels,
-      backward);
+  cct::launch_resize2(x, y, (int64_t)batch * (height / 2), width / 2, channels, 1, !backward,
+                      reinterpret_cast<cudaStream_t>(stream));
   return net_launch_check();
 }
 
 int cct_net_upsample2(const void* x, void* y, int32_t batch, int32_t height, int32_t width, int32_t channels,
                       int32_t backward, void* stream) {
   CCT_REQUIRE(x && y && batch > 0 && height > 0 && width > 0 && channels > 0, "bad upsample2 arguments");
-  const int64_t n = (int64_t)batch * height * width * channels;
-  cct::upsample2_kernel<<<cct::ew_blocks(n), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<__nv_bfloat16*>(y), batch, height, width, channels,
-      backward);
+  cct::launch_resize2(x, y, (int64_t)batch * height, width, channels, 0, backward != 0,
+                      reinterpret_cast<cudaStream_t>(stream));
   return net_launch_check();
 }
 
 int cct_net_add(const void* a, const void* b, void* out, int64_t count, void* stream) {
   CCT_REQUIRE(a && b && out && count > 0, "bad add arguments");
-  cct::add_kernel<<<cct::ew_blocks(count), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(a), reinterpret_cast<const __nv_bfloat16*>(b),
-      reinterpret_cast<__nv_bfloat16*>(out), count);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const __nv_bfloat16 *pa = reinterpret_cast<const __nv_bfloat16*>(a), *pb = reinterpret_cast<const __nv_bfloat16*>(b);
+  __nv_bfloat16* po = reinterpret_cast<__nv_bfloat16*>(out);
+  if (cct::ew_wide(a, b, out, count)) {
+    cct::add_kernel<8><<<cct::ew_blocks(count / 8), 256, 0, st>>>(pa, pb, po, count);
+  } else {
+    cct::add_kernel<1><<<cct::ew_blocks(count), 256, 0, st>>>(pa, pb, po, count);
+  }
   return net_launch_check();
 }
 
 int cct_net_bias_grad(const void* dy, float* db, int64_t pixels, int32_t channels, void* stream) {
   CCT_REQUIRE(dy && db && pixels > 0 && channels > 0, "bad bias_grad arguments");
-  dim3 grid((unsigned)(pixels < 1024 ? pixels : 1024), (unsigned)((channels + 127) / 128));
-  cct::bias_grad_kernel<<<grid, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(dy), db, pixels, channels);
+  cct::launch_bias_grad(dy, db, pixels, channels, reinterpret_cast<cudaStream_t>(stream));
   return net_launch_check();
 }
 

@@ -22,9 +22,6 @@
 
 #include <cstring>
 
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
 #include "cct_common.cuh"
 #include "cct_internal.cuh"
 
@@ -1288,22 +1285,6 @@ void launch_psf(const FpArgs& a, const float* psf, int psf_len, cudaStream_t st)
 // ------------------------------------------------------------------------------------------
 // Launchers
 // ------------------------------------------------------------------------------------------
-
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no libcuda link needed)
-static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess) {
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    }
-  }
-  return fn;
-}
 
 // 3-D tiled map over `images` row-major n x n images with a 96 x 104 box.
 static bool make_box_map(CUtensorMap* map, const void* base, int n, int64_t images, bool bf16) {

@@ -9,11 +9,10 @@
 // and AttenuationVolume (corrct: src/corrct/physics/attenuation.py:105-180) multiplies the
 // incident factor by the mean over sub-angles of the emitted factor of every detector.
 //
-// Phase 1 (maps_scan_kernel): one thread per rotated-frame column c' of one rotation job
-// walks r' = 0..P-1, sampling U only where the column crosses the image (elsewhere U is
-// exactly 0; where all four taps are inside the image, without per-tap tests), keeping the
-// running sum in FP64, and writes W (FP32) to the workspace.
-// Phase 2 (maps_resample_kernel): one thread per map pixel samples W of the incident job
+// Phase 1 (maps_scan_kernel): CTAs of 64 rotated-frame columns c' of one rotation job walk the
+// rows r' where the columns cross the image (elsewhere U is exactly 0), sampling U from staged
+// boxes of mu and keeping the running sums in FP64, and write W (FP32) to the workspace.
+// Phase 2 (maps_resample_kernel): one thread per four map pixels samples W of the incident job
 // and of every emitted (detector, sub-angle) job at the rotated-back position, and writes
 // exp(-L_in) * mean_k exp(-L_out,k) as FP32 or BF16.  Angles are processed in passes sized
 // to the caller's workspace.
@@ -43,8 +42,11 @@ struct MapsPass {
   float emitted_scale;        // quads: mu_out = emitted_scale * mu_in
   const float* mu_in;         // [S][n][n]
   const float* mu_out;
-  const float* mu_in_t;       // [S][n][n] transposed copies (mu_t[s][x][y] = mu[s][y][x]) or NULL
+  const float* mu_in_t;       // [S][n][pitch] transposed copies (mu_t[s][x][y] = mu[s][y][x]) or NULL
   const float* mu_out_t;
+  const float* mu_in_p;       // [S][n][pitch] row-major copies with rows on 16 bytes (n % 4 != 0) or NULL
+  const float* mu_out_p;
+  int pitch;                  // row pitch of the copies: n rounded up to 4, zeros past n
   float* work;                // [S][na][jobs_per_angle][P][P]
   float* kcol;                // [S][na][jobs_per_angle][P] per-column constants of the partner scans
   void* maps;                 // [S][A][D][n][n]
@@ -97,124 +99,40 @@ __device__ __forceinline__ float bilin_zero(const float* img, int h, int w, floa
   return fmaf(fy.f, bot - top, top);
 }
 
-// Bilinear sample whose four taps are known to lie inside the (w x hgt) image.  The clamps are
-// no-ops for such coordinates; they only keep every access in bounds.  Same arithmetic as
-// bilin_zero.
-__device__ __forceinline__ float bilin_inside(const float* img, int w, int hgt, float x, float y) {
-  const FloorSplit fx = floor_split(x), fy = floor_split(y);
-  const int x0 = min(max(fx.i, 0), w - 2), y0 = min(max(fy.i, 0), hgt - 2);
-  const float* q = img + (int64_t)y0 * w + x0;
-  const float v00 = __ldg(q), v01 = __ldg(q + 1), v10 = __ldg(q + w), v11 = __ldg(q + w + 1);
-  const float top = fmaf(fx.f, v01 - v00, v00);
-  const float bot = fmaf(fx.f, v11 - v10, v10);
-  return fmaf(fy.f, bot - top, top);
+// The position (x, y) in packed FP32x2 arithmetic, split like floor_split: fractions, and the index
+// floor(y) * pitch + floor(x) (TR: floor(x) * pitch + floor(y)) of its first tap.
+struct TapSplit {
+  float2 f;
+  unsigned q;
+};
+template <bool TR>
+__device__ __forceinline__ TapSplit tap_split(float2 xy, unsigned pitch) {
+  const float2 t = __fadd2_rd(xy, make_float2(12582912.0f, 12582912.0f));  // 1.5 * 2^23, see floor_split
+  TapSplit r;
+  r.f = __ffma2_rn(__fadd2_rn(t, make_float2(-12582912.0f, -12582912.0f)), make_float2(-1.f, -1.f), xy);
+  const unsigned major = __float_as_uint(TR ? t.x : t.y), minor = __float_as_uint(TR ? t.y : t.x);
+  r.q = major * pitch + (minor - 0x4B400000u * (pitch + 1u));
+  return r;
 }
 
-// The same two samplers on an n x n image whose element (y, x) sits at y * sy + x * sx: row-major
-// (sy, sx) = (n, 1) or transposed (1, n).  The taps and the arithmetic are those of bilin_zero /
-// bilin_inside, so both layouts give bit-identical samples; the layout only decides which lanes
-// of a warp share memory sectors.
-__device__ __forceinline__ float bilin_zero_mu(const float* img, int n, int sy, int sx, float x, float y) {
-  const FloorSplit fx = floor_split(x), fy = floor_split(y);
-  const int x0 = fx.i, y0 = fy.i;
-  const bool xin0 = x0 >= 0 && x0 < n, xin1 = x0 + 1 >= 0 && x0 + 1 < n;
-  const bool yin0 = y0 >= 0 && y0 < n, yin1 = y0 + 1 >= 0 && y0 + 1 < n;
-  const int64_t q = (int64_t)y0 * sy + (int64_t)x0 * sx;
-  const float v00 = (yin0 && xin0) ? __ldg(img + q) : 0.f;
-  const float v01 = (yin0 && xin1) ? __ldg(img + q + sx) : 0.f;
-  const float v10 = (yin1 && xin0) ? __ldg(img + q + sy) : 0.f;
-  const float v11 = (yin1 && xin1) ? __ldg(img + q + sx + sy) : 0.f;
-  const float top = fmaf(fx.f, v01 - v00, v00);
-  const float bot = fmaf(fx.f, v11 - v10, v10);
-  return fmaf(fy.f, bot - top, top);
-}
-
-__device__ __forceinline__ float bilin_inside_mu(const float* img, int n, int sy, int sx, float x, float y) {
-  const FloorSplit fx = floor_split(x), fy = floor_split(y);
-  const int x0 = min(max(fx.i, 0), n - 2), y0 = min(max(fy.i, 0), n - 2);
-  const float* q = img + (y0 * sy + x0 * sx);  // < n * n
-  const float v00 = __ldg(q), v01 = __ldg(q + sx), v10 = __ldg(q + sy), v11 = __ldg(q + sx + sy);
-  const float top = fmaf(fx.f, v01 - v00, v00);
-  const float bot = fmaf(fx.f, v11 - v10, v10);
-  return fmaf(fy.f, bot - top, top);
-}
-
-// Bilinear sample of a (P x P) image with zero outside: one range test picks the unchecked
-// four-tap load for interior coordinates, bilin_zero otherwise.
-__device__ __forceinline__ float bilin_square(const float* img, int P, float x, float y) {
-  const FloorSplit fx = floor_split(x), fy = floor_split(y);
-  if ((unsigned)fx.i < (unsigned)(P - 1) && (unsigned)fy.i < (unsigned)(P - 1)) {
-    const float* q = img + (int64_t)fy.i * P + fx.i;
-    const float v00 = __ldg(q), v01 = __ldg(q + 1), v10 = __ldg(q + P), v11 = __ldg(q + P + 1);
-    const float top = fmaf(fx.f, v01 - v00, v00);
-    const float bot = fmaf(fx.f, v11 - v10, v10);
-    return fmaf(fy.f, bot - top, top);
+// Bilinear sample at xy of a (P x P) image W, and with PAIR of the partner field K[c] - W[r][c]: the
+// x-interpolated column constant minus the sample (bilinear interpolation is linear and K does not vary
+// along rows).  A map pixel rotated about the frame's centre stays 0.2 pixels inside the frame
+// (P >= sqrt(2) n), so its four taps are there; the minimum keeps the loads of pixels past the image
+// edge, which are not stored, in bounds.
+template <bool PAIR>
+__device__ __forceinline__ void bilin_frame(const float* img, const float* K, unsigned P, float2 xy, float* La, float* Lb) {
+  const TapSplit t = tap_split<false>(xy, P);
+  const float *p = img + min(t.q, P * P - P - 2u), *q = p + P;
+  const float v00 = __ldg(p), v01 = __ldg(p + 1), v10 = __ldg(q), v11 = __ldg(q + 1);
+  const float top = fmaf(t.f.x, v01 - v00, v00);
+  const float bot = fmaf(t.f.x, v11 - v10, v10);
+  *La = fmaf(t.f.y, bot - top, top);
+  if constexpr (PAIR) {
+    const unsigned c = min((unsigned)floor_split(xy.x).i, P - 2u);
+    const float k0 = __ldg(K + c), k1 = __ldg(K + c + 1);
+    *Lb = fmaf(t.f.x, k1 - k0, k0) - *La;
   }
-  return bilin_zero(img, P, P, x, y);
-}
-
-// Bilinear samples at (x, y) of a (P x P) image W and of the partner field K[c] - W[r][c]
-// (zero outside the frame for both).  *La is bilin_square(W) exactly.  Inside the frame the
-// partner's sample is the x-interpolated column constant minus *La (bilinear interpolation is
-// linear and K does not vary along rows); at the frame edge, where the partner field is zero
-// outside, its four taps are interpolated.
-__device__ __forceinline__ void bilin_square_pair(const float* img, const float* K, int P, float x, float y,
-                                                  float* La, float* Lb) {
-  const FloorSplit fx = floor_split(x), fy = floor_split(y);
-  const int x0 = fx.i, y0 = fy.i;
-  float v00, v01, v10, v11, u00, u01, u10, u11;
-  if ((unsigned)x0 < (unsigned)(P - 1) && (unsigned)y0 < (unsigned)(P - 1)) {
-    const float* q = img + (int64_t)y0 * P + x0;
-    v00 = __ldg(q); v01 = __ldg(q + 1); v10 = __ldg(q + P); v11 = __ldg(q + P + 1);
-    const float k0 = __ldg(K + x0), k1 = __ldg(K + x0 + 1);
-    const float top = fmaf(fx.f, v01 - v00, v00);
-    const float bot = fmaf(fx.f, v11 - v10, v10);
-    *La = fmaf(fy.f, bot - top, top);
-    *Lb = fmaf(fx.f, k1 - k0, k0) - *La;
-    return;
-  } else {
-    const bool xin0 = x0 >= 0 && x0 < P, xin1 = x0 + 1 >= 0 && x0 + 1 < P;
-    const bool yin0 = y0 >= 0 && y0 < P, yin1 = y0 + 1 >= 0 && y0 + 1 < P;
-    const float k0 = xin0 ? __ldg(K + x0) : 0.f, k1 = xin1 ? __ldg(K + x0 + 1) : 0.f;
-    v00 = (yin0 && xin0) ? __ldg(img + (int64_t)y0 * P + x0) : 0.f;
-    v01 = (yin0 && xin1) ? __ldg(img + (int64_t)y0 * P + x0 + 1) : 0.f;
-    v10 = (yin1 && xin0) ? __ldg(img + (int64_t)(y0 + 1) * P + x0) : 0.f;
-    v11 = (yin1 && xin1) ? __ldg(img + (int64_t)(y0 + 1) * P + x0 + 1) : 0.f;
-    u00 = (yin0 && xin0) ? k0 - v00 : 0.f;
-    u01 = (yin0 && xin1) ? k1 - v01 : 0.f;
-    u10 = (yin1 && xin0) ? k0 - v10 : 0.f;
-    u11 = (yin1 && xin1) ? k1 - v11 : 0.f;
-  }
-  const float top = fmaf(fx.f, v01 - v00, v00);
-  const float bot = fmaf(fx.f, v11 - v10, v10);
-  *La = fmaf(fy.f, bot - top, top);
-  const float topb = fmaf(fx.f, u01 - u00, u00);
-  const float botb = fmaf(fx.f, u11 - u10, u10);
-  *Lb = fmaf(fy.f, botb - topb, topb);
-}
-
-// Integer r in [*lo, *hi] with x(r) = ax + r bx and y(r) = ay + r by both in [lim0, lim1]
-// (exact arithmetic), clipped to [0, P - 1]; *lo > *hi when there is none.
-__device__ __forceinline__ void column_inside(double ax, double bx, double ay, double by, double lim0, double lim1,
-                                              int P, int* lo, int* hi) {
-  double tlo = -1e300, thi = 1e300;
-  if (fabs(bx) < 1e-12) {
-    if (!(ax >= lim0 && ax <= lim1)) { *lo = 1; *hi = 0; return; }
-  } else {
-    double t0 = (lim0 - ax) / bx, t1 = (lim1 - ax) / bx;
-    if (t0 > t1) { double t = t0; t0 = t1; t1 = t; }
-    tlo = fmax(tlo, t0); thi = fmin(thi, t1);
-  }
-  if (fabs(by) < 1e-12) {
-    if (!(ay >= lim0 && ay <= lim1)) { *lo = 1; *hi = 0; return; }
-  } else {
-    double t0 = (lim0 - ay) / by, t1 = (lim1 - ay) / by;
-    if (t0 > t1) { double t = t0; t0 = t1; t1 = t; }
-    tlo = fmax(tlo, t0); thi = fmin(thi, t1);
-  }
-  if (tlo > thi) { *lo = 1; *hi = 0; return; }
-  *lo = (int)fmax(0.0, ceil(tlo));
-  *hi = (int)fmin((double)(P - 1), floor(thi));
 }
 
 // Range of r' (inclusive) where the column c' samples inside (-1, n) x (-1, n) of mu, widened
@@ -243,16 +161,178 @@ __device__ __forceinline__ void column_support(double ax, double bx, double ay, 
   *hi = min(P - 1, (int)ceil(thi) + 1);
 }
 
-// One thread per column; the 32 columns of a warp walk the rows in lockstep (coalesced W
-// stores), with warp-uniform row ranges: no lane samples before the warp's first support row or
-// after its last, and rows where every lane's four taps are inside mu skip the per-tap tests.
+// ------------------------------------------------------------------------------------------
+// Scan
+//
+// A CTA owns 64 rotated-frame columns of one job and walks their support rows in chunks of 64.  The
+// bounding box of a chunk in mu (at most 94 x 100 pixels, zeros outside the image) is staged in
+// shared memory; each of 256 threads then samples 16 consecutive rows of one column, the column's four
+// threads exchange their FP64 sums, and each writes its rows.  A warp is 32 neighbouring columns at
+// one row, so the stores of W are coalesced; where the columns run closer to y than to x the box comes
+// from the transposed copy of mu, and the row stride of 128 floats makes a tap's bank its
+// position along the columns (1.6 wavefronts per load on average).
+//
+// Bound: sampling mu directly, a warp's load touched ~10 cache lines and the tag stage of L1, not its
+// data, set the pace; staged, a row costs ~12 data wavefronts.  (8 slices of 512^2, 14 jobs per
+// slice: 188 us per launch sampling directly, 121 us so.)  Staging needs rows on 16-byte boundaries:
+// with n % 4 != 0 the row-major side also comes from a copy with padded rows (301^2: 187 us per launch
+// with 4-byte staging, 117 us so).
+// ------------------------------------------------------------------------------------------
+constexpr int SCAN_COLS = 64;
+constexpr int SCAN_ROWS = 64;
+constexpr int SCAN_THREADS = 256;
+constexpr int SCAN_PER_THREAD = SCAN_ROWS / (SCAN_THREADS / SCAN_COLS);  // rows of one thread per chunk
+constexpr int SCAN_STRIDE = 128;
+constexpr int SCAN_BOX_W = 100, SCAN_BOX_H = 94;
+constexpr size_t SCAN_SMEM = SCAN_BOX_H * SCAN_STRIDE * sizeof(float) + 4 * SCAN_COLS * sizeof(double);
+
+// Raised (never trapped) if a chunk's box would exceed its bound; rotation matrices cannot reach it.
+__device__ int g_scan_overflow = 0;
+
+// Stage a box in items of W pixels (W = 4: pitch, bu and the address allow 16-byte loads, and the
+// pitch's pixels past n are zeros), BATCH items' loads in flight per thread.
+template <int W, int BATCH>
+__device__ __forceinline__ void scan_stage(float* z, const float* mu, int n, int pitch, int bu, int bv, int bw, int bh,
+                                           int tid) {
+  const int per_row = (bw + W - 1) / W, items = per_row * bh;
+  // it / per_row = (it * ceil(2^20 / per_row)) >> 20, exact while it * per_row < 2^20
+  const unsigned magic = (1048576u + (unsigned)per_row - 1u) / (unsigned)per_row;
+  for (int base = tid; base < items; base += SCAN_THREADS * BATCH) {
+    float v[BATCH][W];
+#pragma unroll
+    for (int k = 0; k < BATCH; ++k) {
+      const int it = base + k * SCAN_THREADS;
+      const int row = (int)(((unsigned)it * magic) >> 20);
+      const int gv = bv + row, gu = bu + W * (it - row * per_row);
+#pragma unroll
+      for (int q = 0; q < W; ++q) v[k][q] = 0.f;
+      if (it < items && (unsigned)gv < (unsigned)n && (unsigned)gu < (unsigned)n) {
+        const float* src = mu + (gv * pitch + gu);
+        if constexpr (W == 4) {
+          const float4 t = __ldg(reinterpret_cast<const float4*>(src));
+          v[k][0] = t.x; v[k][1] = t.y; v[k][2] = t.z; v[k][3] = t.w;
+        } else {
+          v[k][0] = __ldg(src);
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < BATCH; ++k) {
+      const int it = base + k * SCAN_THREADS;
+      const int row = (int)(((unsigned)it * magic) >> 20);
+      if (it >= items) break;
+      float* dst = z + (row * SCAN_STRIDE + W * (it - row * per_row));
+      if constexpr (W == 4) {
+        *reinterpret_cast<float4*>(dst) = make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
+      } else {
+        *dst = v[k][0];
+      }
+    }
+  }
+}
+
+// The walk of one band.  (u, v) = (x, y), or (y, x) with TR: u runs along the staged rows.
+template <bool PAIRS, bool TR>
+__device__ __forceinline__ void scan_band(const MapsPass& p, float* z, double* sums, const float* mu, int pitch, const float* mu_row,
+                                          float m00, float m01, float m02, float m10, float m11, float m12, int c0,
+                                          int blo, int bhi, float* W, float* kcol) {
+  const int n = p.n, P = p.P;
+  const int tid = threadIdx.x;
+  const int col = tid & (SCAN_COLS - 1), quarter = tid / SCAN_COLS;
+  const int c = min(c0 + col, P - 1);
+  const bool valid = c0 + col < P;  // lanes past the frame shadow the last column, store nothing
+  const float fc = (float)c, fc1 = (float)min(c0 + SCAN_COLS - 1, P - 1);
+  const float xc = fmaf(m00, fc, m02), yc = fmaf(m10, fc, m12);
+  // wrap-around term U[P-1] / 2 of roll + cumsum (0 unless the support reaches the last row)
+  double wrap = 0.0;
+  if (bhi == P - 1) {
+    const float fr = (float)(P - 1);
+    wrap = 0.5 * (double)bilin_zero(mu_row, n, n, fmaf(m01, fr, xc), fmaf(m11, fr, yc));
+  }
+  const bool vec4 = pitch % 4 == 0 && (reinterpret_cast<uintptr_t>(mu) & 15) == 0;
+  double carry = 0.0;
+  for (int r0 = blo; r0 <= bhi; r0 += SCAN_ROWS) {
+    const int r_last = min(r0 + SCAN_ROWS - 1, bhi);
+    // box of the chunk's samples, widened by the taps; u origin a multiple of 4
+    const float fr0 = (float)r0, fr1 = (float)r_last;
+    const float xa = fmaf(m00, (float)c0, m02), xb = fmaf(m00, fc1, m02);
+    const float ya = fmaf(m10, (float)c0, m12), yb = fmaf(m10, fc1, m12);
+    const float x0 = fmaf(m01, fr0, xa), x1 = fmaf(m01, fr0, xb), x2 = fmaf(m01, fr1, xa), x3 = fmaf(m01, fr1, xb);
+    const float y0 = fmaf(m11, fr0, ya), y1 = fmaf(m11, fr0, yb), y2 = fmaf(m11, fr1, ya), y3 = fmaf(m11, fr1, yb);
+    const float xmin = fminf(fminf(x0, x1), fminf(x2, x3)), xmax = fmaxf(fmaxf(x0, x1), fmaxf(x2, x3));
+    const float ymin = fminf(fminf(y0, y1), fminf(y2, y3)), ymax = fmaxf(fmaxf(y0, y1), fmaxf(y2, y3));
+    const int bu = ((int)floorf(TR ? ymin : xmin) - 1) & ~3, bu1 = (int)floorf(TR ? ymax : xmax) + 2;
+    const int bv = (int)floorf(TR ? xmin : ymin) - 1, bv1 = (int)floorf(TR ? xmax : ymax) + 2;
+    const int bw = bu1 - bu + 1, bh = bv1 - bv + 1;
+    if (bw > SCAN_BOX_W + 3 || bh > SCAN_BOX_H) {  // uniform; never trap
+      if (tid == 0) atomicExch(&g_scan_overflow, 1);
+      return;
+    }
+    if (vec4) {
+      scan_stage<4, 3>(z, mu, n, pitch, bu, bv, bw, bh, tid);
+    } else {
+      scan_stage<1, 10>(z, mu, n, pitch, bu, bv, bw, bh, tid);
+    }
+    __syncthreads();
+
+    // this thread's rows: samples as bilin_zero forms them (taps outside mu are staged zeros)
+    const int rb = r0 + SCAN_PER_THREAD * quarter;
+    const int rows = min(max(r_last - rb + 1, 0), SCAN_PER_THREAD);
+    const unsigned zoff = (unsigned)(-bv * SCAN_STRIDE - bu);
+    const float2 m = make_float2(m01, m11), c2 = make_float2(xc, yc);
+    float u[SCAN_PER_THREAD];
+    double sum = 0.0;
+#pragma unroll
+    for (int k = 0; k < SCAN_PER_THREAD; ++k) {
+      u[k] = 0.f;
+      if (k < rows) {  // uniform in a warp
+        const float fr = (float)(rb + k);
+        const TapSplit t = tap_split<TR>(__ffma2_rn(m, make_float2(fr, fr), c2), SCAN_STRIDE);
+        const float* q = z + (int)(t.q + zoff);
+        const float v00 = q[0], v01 = TR ? q[SCAN_STRIDE] : q[1], v10 = TR ? q[1] : q[SCAN_STRIDE], v11 = q[SCAN_STRIDE + 1];
+        const float top = fmaf(t.f.x, v01 - v00, v00);
+        const float bot = fmaf(t.f.x, v11 - v10, v10);
+        u[k] = fmaf(t.f.y, bot - top, top);
+        sum += (double)u[k];
+      }
+    }
+    sums[quarter * SCAN_COLS + col] = sum;
+    __syncthreads();
+    // W[r] = sum_{k<r} U[k] + U[r]/2 + wrap in FP64
+    double acc = carry;
+#pragma unroll
+    for (int q = 0; q < SCAN_THREADS / SCAN_COLS; ++q) {
+      const double sq = sums[q * SCAN_COLS + col];
+      if (q < quarter) acc += sq;
+      carry += sq;
+    }
+    float* w = W + (int64_t)rb * P + c;
+#pragma unroll
+    for (int k = 0; k < SCAN_PER_THREAD; ++k) {
+      if (k < rows) {
+        const double d = (double)u[k];
+        if (valid) *w = (float)(fma(0.5, d, acc) + wrap);
+        acc += d;
+        w += P;
+      }
+    }
+  }
+  if (PAIRS && kcol != nullptr && quarter == 0 && valid) {
+    // the partner angle (phi + pi) rotates by a half turn more: its frame is this one turned
+    // about the centre, and its W at this frame's (r', c') is K[c'] - W[r'][c'] with
+    // K = sum_k U[k] + U[0]/2 + U[P-1]/2 (the reverse roll + cumsum of the same column)
+    const double first = blo == 0 ? 0.5 * (double)bilin_zero(mu_row, n, n, xc, yc) : 0.0;
+    kcol[c] = (float)(carry + first + wrap);
+  }
+}
+
 template <bool PAIRS>
-__global__ void __launch_bounds__(128) maps_scan_kernel(MapsPass p) {
+__global__ void __launch_bounds__(SCAN_THREADS, 4) maps_scan_kernel(MapsPass p) {
+  extern __shared__ __align__(16) float scan_z[];
+  double* sums = reinterpret_cast<double*>(scan_z + SCAN_BOX_H * SCAN_STRIDE);
   const int P = p.P, n = p.n;
-  const int cpr_raw = blockIdx.x * blockDim.x + threadIdx.x;  // rotated-frame column c'
-  const bool valid = cpr_raw < P;
-  const int cpr = valid ? cpr_raw : P - 1;  // lanes past the frame shadow the last column, store nothing
-  const int job_lin = blockIdx.y;           // (angle in pass, job)
+  const int c0 = blockIdx.x * SCAN_COLS;
+  const int job_lin = blockIdx.y;  // (angle in pass, job)
   const int s = blockIdx.z;
   const int ai = job_lin / p.jobs_per_angle;
   const int job = job_lin - ai * p.jobs_per_angle;
@@ -261,89 +341,47 @@ __global__ void __launch_bounds__(128) maps_scan_kernel(MapsPass p) {
   if (a < 0) return;  // the whole CTA
   const double* Md = job_matrix(p, a, job, 0);  // rotate(-phi)
   const bool incident = p.has_in && job == 0;
-  // the lanes of a warp step along (m00, m10) in mu: where that is closer to y than to x, the
-  // transposed copy (if given) puts neighbouring lanes in neighbouring memory
+  // neighbouring columns step along (m00, m10) in mu
   const float* mu_t = incident ? p.mu_in_t : p.mu_out_t;
   const bool tr = mu_t != nullptr && fabs(Md[3]) > fabs(Md[0]);
-  const float* mu = (tr ? mu_t : (incident ? p.mu_in : p.mu_out)) + (int64_t)s * n * n;
-  const int sy = tr ? 1 : n, sx = tr ? n : 1;  // element (y, x) of mu at y * sy + x * sx
+  const float* mu_row = (incident ? p.mu_in : p.mu_out) + (int64_t)s * n * n;
   // mu coordinates = padded coordinates - e
   const float m00 = (float)Md[0], m01 = (float)Md[1], m02 = (float)(Md[2] - p.e);
   const float m10 = (float)Md[3], m11 = (float)Md[4], m12 = (float)(Md[5] - p.e);
-  const double ax = Md[0] * cpr + Md[2] - p.e, ay = Md[3] * cpr + Md[5] - p.e;
-  int lo, hi;
-  column_support(ax, Md[1], ay, Md[4], n, P, &lo, &hi);
-  if (lo > hi) { lo = P; hi = -1; }
-  // rows whose four taps all lie inside mu, with a 0.01-pixel margin against the FP32
-  // evaluation of the coordinates below
-  int ilo = P, ihi = -1;
-  if (n >= 2) column_inside(ax, Md[1], ay, Md[4], 0.01, (double)n - 1.01, P, &ilo, &ihi);
-  ilo = max(ilo, lo);
-  ihi = min(ihi, hi);
-  if (ilo > ihi) { ilo = P; ihi = -1; }
-  int wlo = lo, whi = hi, wilo = ilo, wihi = ihi;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    wlo = min(wlo, __shfl_xor_sync(0xffffffffu, wlo, o));
-    whi = max(whi, __shfl_xor_sync(0xffffffffu, whi, o));
-    wilo = max(wilo, __shfl_xor_sync(0xffffffffu, wilo, o));
-    wihi = min(wihi, __shfl_xor_sync(0xffffffffu, wihi, o));
-  }
-  if (wilo > wihi) { wilo = whi + 1; wihi = whi; }  // no row is inside for every lane
-  const float fc = (float)cpr;
-  const float xc = fmaf(m00, fc, m02), yc = fmaf(m10, fc, m12);
-  float* W = p.work + (((int64_t)s * p.na + ai) * p.jobs_per_angle + job) * (int64_t)P * P + cpr;
-
-  // wrap-around term U[P-1] / 2 of roll + cumsum
-  double wrap = 0.0;
-  if (P - 1 >= lo && P - 1 <= hi) {
-    const float fr = (float)(P - 1);
-    wrap = 0.5 * (double)bilin_zero_mu(mu, n, sy, sx, fmaf(m01, fr, xc), fmaf(m11, fr, yc));
-  }
-  // W[r] = acc + U[r]/2 + wrap with acc = sum_{k<r} U[k] (FP64); U = 0 outside [lo, hi].  Only
-  // the warp's rows [wlo, whi] are stored: outside them W is constant per column and the
-  // resample, whose positions all map back into the image, never reads it there
-  // (tests/test_host.py::test_maps_resample_reads_only_scanned_rows mirrors that arithmetic).
-  double acc = 0.0;
-  int r = wlo;
-  for (; r < wilo; ++r) {
-    const float fr = (float)r;
-    const float u = (r >= lo && r <= hi) ? bilin_zero_mu(mu, n, sy, sx, fmaf(m01, fr, xc), fmaf(m11, fr, yc)) : 0.f;
-    if (valid) W[(int64_t)r * P] = (float)(acc + 0.5 * (double)u + wrap);
-    acc += (double)u;
-  }
-  for (; r + 3 <= wihi; r += 4) {
-    float u[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float fr = (float)(r + k);
-      u[k] = bilin_inside_mu(mu, n, sy, sx, fmaf(m01, fr, xc), fmaf(m11, fr, yc));
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (valid) W[(int64_t)(r + k) * P] = (float)(acc + 0.5 * (double)u[k] + wrap);
-      acc += (double)u[k];
+  // support rows of the band: outside them W is constant per column and the resample, whose positions
+  // all map back into the image, never reads it
+  // (tests/test_host.py::test_maps_resample_reads_only_scanned_rows mirrors that arithmetic)
+  int lo = P, hi = -1;
+  if ((int)threadIdx.x < SCAN_COLS && c0 + (int)threadIdx.x < P) {
+    const int c = c0 + threadIdx.x;
+    column_support(Md[0] * c + Md[2] - p.e, Md[1], Md[3] * c + Md[5] - p.e, Md[4], n, P, &lo, &hi);
+    if (lo > hi) {
+      lo = P;
+      hi = -1;
     }
   }
-  for (; r <= wihi; ++r) {
-    const float fr = (float)r;
-    const float u = bilin_inside_mu(mu, n, sy, sx, fmaf(m01, fr, xc), fmaf(m11, fr, yc));
-    if (valid) W[(int64_t)r * P] = (float)(acc + 0.5 * (double)u + wrap);
-    acc += (double)u;
+  __shared__ int range_sh[2];
+  if (threadIdx.x == 0) {
+    range_sh[0] = P;
+    range_sh[1] = -1;
   }
-  for (; r <= whi; ++r) {
-    const float fr = (float)r;
-    const float u = (r >= lo && r <= hi) ? bilin_zero_mu(mu, n, sy, sx, fmaf(m01, fr, xc), fmaf(m11, fr, yc)) : 0.f;
-    if (valid) W[(int64_t)r * P] = (float)(acc + 0.5 * (double)u + wrap);
-    acc += (double)u;
+  __syncthreads();
+  if (threadIdx.x < SCAN_COLS) {
+    atomicMin(&range_sh[0], lo);
+    atomicMax(&range_sh[1], hi);
   }
-  if (PAIRS && b >= 0 && valid) {
-    // the partner angle (phi + pi) rotates by a half turn more: its frame is this one turned
-    // about the centre, and its W at this frame's (r', c') is K[c'] - W[r'][c'] with
-    // K = sum_k U[k] + U[0]/2 + U[P-1]/2 (the reverse roll + cumsum of the same column)
-    double first = 0.0;
-    if (0 >= lo && 0 <= hi) first = 0.5 * (double)bilin_zero_mu(mu, n, sy, sx, xc, yc);
-    p.kcol[(((int64_t)s * p.na + ai) * p.jobs_per_angle + job) * P + cpr] = (float)(acc + first + wrap);
+  __syncthreads();
+  const int64_t slot = ((int64_t)s * p.na + ai) * p.jobs_per_angle + job;
+  float* W = p.work + slot * (int64_t)P * P;
+  float* kcol = PAIRS && b >= 0 ? p.kcol + slot * P : nullptr;
+  const float* mu_p = incident ? p.mu_in_p : p.mu_out_p;
+  const int64_t copy = (int64_t)s * n * p.pitch;
+  if (tr) {
+    scan_band<PAIRS, true>(p, scan_z, sums, mu_t + copy, p.pitch, mu_row, m00, m01, m02, m10, m11, m12, c0, range_sh[0],
+                           range_sh[1], W, kcol);
+  } else {
+    scan_band<PAIRS, false>(p, scan_z, sums, mu_p != nullptr ? mu_p + copy : mu_row, mu_p != nullptr ? p.pitch : n, mu_row,
+                            m00, m01, m02, m10, m11, m12, c0, range_sh[0], range_sh[1], W, kcol);
   }
 }
 
@@ -388,16 +426,12 @@ __global__ void __launch_bounds__(256, PAIRS ? 5 : 1) maps_resample_kernel(MapsP
     const float* m = rs_mats + job * 6;
     const float* w = wbase + (int64_t)job * P * P;
     const float* kc = kbase + (int64_t)job * P;
+    const float2 my = make_float2(m[1], m[4]);
+    const float2 c0 = make_float2(fmaf(m[0], X, m[2]), fmaf(m[3], X, m[5]));
 #pragma unroll
     for (int k = 0; k < RS_PIX; ++k) {
       const float Y = (float)(i0 + 8 * k + p.e);
-      const float x = fmaf(m[1], Y, fmaf(m[0], X, m[2]));
-      const float y = fmaf(m[4], Y, fmaf(m[3], X, m[5]));
-      if (PAIRS && paired) {
-        bilin_square_pair(w, kc, P, x, y, &L[k], &Lb[k]);
-      } else {
-        L[k] = bilin_square(w, P, x, y);
-      }
+      bilin_frame<PAIRS>(w, kc, (unsigned)P, __ffma2_rn(my, make_float2(Y, Y), c0), &L[k], &Lb[k]);
     }
   };
   auto store4 = [&](int64_t plane, const float* v) {
@@ -439,28 +473,19 @@ __global__ void __launch_bounds__(256, PAIRS ? 5 : 1) maps_resample_kernel(MapsP
     }
     return;
   }
-  float f_in[RS_PIX], f_inb[RS_PIX];
+  // exp(-L_in) mean exp(-L_out): with one emitted direction the exponent is summed first
+  float l_in[RS_PIX], l_inb[RS_PIX];
   int job = 0;
   if (p.has_in) {
-    sample4(0, L, Lb);
-#pragma unroll
-    for (int k = 0; k < RS_PIX; ++k) {
-      f_in[k] = __expf(-L[k]);
-      f_inb[k] = paired ? __expf(-Lb[k]) : 1.f;
-    }
+    sample4(0, l_in, l_inb);
     job = 1;
   } else {
 #pragma unroll
-    for (int k = 0; k < RS_PIX; ++k) f_in[k] = f_inb[k] = 1.f;
+    for (int k = 0; k < RS_PIX; ++k) l_in[k] = l_inb[k] = 0.f;
   }
   for (int d = 0; d < p.n_det; ++d) {
     float f[RS_PIX], fb[RS_PIX];
-#pragma unroll
-    for (int k = 0; k < RS_PIX; ++k) {
-      f[k] = f_in[k];
-      fb[k] = f_inb[k];
-    }
-    if (p.has_out) {
+    if (p.has_out && p.n_sub > 1) {
       float sum[RS_PIX] = {0.f, 0.f, 0.f, 0.f}, sumb[RS_PIX] = {0.f, 0.f, 0.f, 0.f};
       for (int q = 0; q < p.n_sub; ++q) {
         sample4(job + d * p.n_sub + q, L, Lb);
@@ -470,19 +495,23 @@ __global__ void __launch_bounds__(256, PAIRS ? 5 : 1) maps_resample_kernel(MapsP
           if (paired) sumb[k] += __expf(-Lb[k]);
         }
       }
-      if (p.n_sub == 1) {
+      const float ns = (float)p.n_sub;
 #pragma unroll
-        for (int k = 0; k < RS_PIX; ++k) {
-          f[k] *= sum[k];
-          fb[k] *= sumb[k];
-        }
+      for (int k = 0; k < RS_PIX; ++k) {
+        f[k] = __expf(-l_in[k]) * (sum[k] / ns);
+        if (paired) fb[k] = __expf(-l_inb[k]) * (sumb[k] / ns);
+      }
+    } else {
+      if (p.has_out) {
+        sample4(job + d, L, Lb);
       } else {
-        const float ns = (float)p.n_sub;
 #pragma unroll
-        for (int k = 0; k < RS_PIX; ++k) {
-          f[k] *= sum[k] / ns;
-          fb[k] *= sumb[k] / ns;
-        }
+        for (int k = 0; k < RS_PIX; ++k) L[k] = Lb[k] = 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < RS_PIX; ++k) {
+        f[k] = __expf(-(l_in[k] + L[k]));
+        if (paired) fb[k] = __expf(-(l_inb[k] + Lb[k]));
       }
     }
     store4(((int64_t)s * p.n_angles + a) * p.n_det + d, f);
@@ -498,7 +527,9 @@ __global__ void __launch_bounds__(256, PAIRS ? 5 : 1) maps_resample_kernel(MapsP
 // exp(-L[k]) * exp(-emitted_scale * L[src[k]]), src[k] naming which of the four angles the
 // emitted direction of angle k is (its rotation angle differs from the reference's emitted angle
 // only by the float32 rounding of the angles, like a half-turn partner's).  Four maps from two
-// gathers per pixel, where the per-pair resample needs two gathers for two maps.
+// gathers per pixel, where the per-pair resample needs two gathers for two maps.  Bound: the L1 pipe
+// (16 taps of W per pixel), then issue: 56 (slice, quad)s of 512^2 took 158 us with 64-bit index
+// arithmetic, range tests that a pixel of the image cannot fail and two exps per map, 125 us so.
 __global__ void __launch_bounds__(256, 5) maps_resample_quad_kernel(MapsPass p) {
   __shared__ float qm[2][6];  // rotate(+phi) matrices of the two entries' angles
   __shared__ int qa[4];       // the four angles
@@ -540,30 +571,39 @@ __global__ void __launch_bounds__(256, 5) maps_resample_quad_kernel(MapsPass p) 
     const int slot = 2 * qi + w;
     const float* wf = p.work + ((int64_t)s * p.na + slot) * (int64_t)P * P;
     const float* kc = p.kcol + ((int64_t)s * p.na + slot) * (int64_t)P;
+    const float2 my = make_float2(m[1], m[4]);
+    const float2 c0 = make_float2(fmaf(m[0], X, m[2]), fmaf(m[3], X, m[5]));
 #pragma unroll
     for (int k = 0; k < RS_PIX; ++k) {
       const float Y = (float)(i0 + 8 * k + p.e);
-      const float x = fmaf(m[1], Y, fmaf(m[0], X, m[2]));
-      const float y = fmaf(m[4], Y, fmaf(m[3], X, m[5]));
-      bilin_square_pair(wf, kc, P, x, y, &L[2 * w][k], &L[2 * w + 1][k]);
+      bilin_frame<true>(wf, kc, (unsigned)P, __ffma2_rn(my, make_float2(Y, Y), c0), &L[2 * w][k], &L[2 * w + 1][k]);
     }
   }
+  // exp(-L[q]) exp(-scale L[source]) with the exponents summed first (one exp per map and pixel)
+  auto emit = [&](int q, const float (&lq)[RS_PIX], const float (&le)[RS_PIX]) {
+    const int64_t off = ((int64_t)s * p.n_angles + qa[q]) * n2 + (int64_t)i0 * n + j;  // n_det == 1
+#pragma unroll
+    for (int k = 0; k < RS_PIX; ++k) {
+      if (i0 + 8 * k >= n) break;
+      const float v = __expf(-fmaf(sc, le[k], lq[k]));
+      if (p.maps_dtype == CCT_DTYPE_BF16) {
+        reinterpret_cast<__nv_bfloat16*>(p.maps)[off + (int64_t)8 * k * n] = __float2bfloat16_rn(v);
+      } else {
+        reinterpret_cast<float*>(p.maps)[off + (int64_t)8 * k * n] = v;
+      }
+    }
+  };
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const int src = qs[q];
-    const int64_t plane = (int64_t)s * p.n_angles + qa[q];  // n_det == 1
-#pragma unroll
-    for (int k = 0; k < RS_PIX; ++k) {
-      const int i = i0 + 8 * k;
-      if (i >= n) break;
-      const float le = src == 0 ? L[0][k] : (src == 1 ? L[1][k] : (src == 2 ? L[2][k] : L[3][k]));
-      const float v = __expf(-L[q][k]) * __expf(-sc * le);
-      const int64_t off = plane * n2 + (int64_t)i * n + j;
-      if (p.maps_dtype == CCT_DTYPE_BF16) {
-        reinterpret_cast<__nv_bfloat16*>(p.maps)[off] = __float2bfloat16_rn(v);
-      } else {
-        reinterpret_cast<float*>(p.maps)[off] = v;
-      }
+    if (src == 0) {
+      emit(q, L[q], L[0]);
+    } else if (src == 1) {
+      emit(q, L[q], L[1]);
+    } else if (src == 2) {
+      emit(q, L[q], L[2]);
+    } else {
+      emit(q, L[q], L[3]);
     }
   }
 }
@@ -575,39 +615,63 @@ int padded_edge(int n) {
 }
 
 // mu_t[s][x][y] = mu[s][y][x] for the scan's transposed reads (32 x 32 tiles through shared
-// memory, coalesced on both sides).
+// memory, coalesced on both sides), rows of `pitch` with zeros past n.
 __global__ void __launch_bounds__(256) maps_transpose_kernel(const float* __restrict__ src, float* __restrict__ dst,
-                                                             int n) {
+                                                             int n, int pitch) {
   __shared__ float t[32][33];
-  const int64_t off = (int64_t)blockIdx.z * n * n;
+  src += (int64_t)blockIdx.z * n * n;
+  dst += (int64_t)blockIdx.z * n * pitch;
   const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
   for (int k = threadIdx.y; k < 32; k += 8) {
     const int y = y0 + k, x = x0 + threadIdx.x;
-    if (y < n && x < n) t[k][threadIdx.x] = src[off + (int64_t)y * n + x];
+    t[k][threadIdx.x] = y < n && x < n ? src[(int64_t)y * n + x] : 0.f;
   }
   __syncthreads();
   for (int k = threadIdx.y; k < 32; k += 8) {
     const int x = x0 + k, y = y0 + threadIdx.x;
-    if (x < n && y < n) dst[off + (int64_t)x * n + y] = t[threadIdx.x][k];
+    if (x < n && y < pitch) dst[(int64_t)x * pitch + y] = t[threadIdx.x][k];
   }
 }
 
-static size_t transposed_bytes(const cct_maps_desc* d) {
-  const size_t b = (size_t)d->n * d->n * sizeof(float) * d->n_slices;
+// Row-major copy with rows of `pitch`, zeros past n.
+__global__ void __launch_bounds__(256) maps_pad_kernel(const float* __restrict__ src, float* __restrict__ dst, int n,
+                                                       int pitch) {
+  const int64_t row = blockIdx.y + (int64_t)blockIdx.z * n;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x < pitch) dst[row * pitch + x] = x < n ? src[row * n + x] : 0.f;
+}
+
+static int copy_pitch(int n) { return (n + 3) & ~3; }
+
+// One copy of mu in the workspace's prefix: transposed, or (n % 4 != 0) with padded rows.
+static size_t copy_bytes(const cct_maps_desc* d) {
+  const size_t b = (size_t)d->n * copy_pitch(d->n) * sizeof(float) * d->n_slices;
   return (b + 255) & ~(size_t)255;
 }
 
-static void launch_transpose(const float* src, float* dst, int n, int slices, cudaStream_t st) {
-  const int t = (n + 31) / 32;
-  maps_transpose_kernel<<<dim3(t, t, slices), dim3(32, 8), 0, st>>>(src, dst, n);
+// Transposed (and padded) copies of mu at *work, which moves past them.
+static void launch_copies(const cct_maps_desc* d, const float* mu, char** work, const float** mu_t, const float** mu_p,
+                          cudaStream_t st) {
+  const int n = d->n, pitch = copy_pitch(n), t = (n + 31) / 32;
+  float* dst = reinterpret_cast<float*>(*work);
+  maps_transpose_kernel<<<dim3(t, t, d->n_slices), dim3(32, 8), 0, st>>>(mu, dst, n, pitch);
+  *mu_t = dst;
+  *work += copy_bytes(d);
+  if (pitch != n) {
+    dst = reinterpret_cast<float*>(*work);
+    maps_pad_kernel<<<dim3((pitch + 255) / 256, n, d->n_slices), 256, 0, st>>>(mu, dst, n, pitch);
+    *mu_p = dst;
+    *work += copy_bytes(d);
+  }
 }
 
-// Entries per pass and whether the workspace also holds `copies` transposed copies of mu at its
-// start: they are used when, after them, at least half the entries of a pass without them fit.
-static int plan_pass(const cct_maps_desc* d, size_t work_bytes, int64_t per_entry, int entries, int copies,
+// Entries per pass and whether the workspace also holds the copies of `volumes` attenuation volumes at
+// its start: they are used when, after them, at least half the entries of a pass without them fit.
+static int plan_pass(const cct_maps_desc* d, size_t work_bytes, int64_t per_entry, int entries, int volumes,
                      size_t* prefix) {
+  const int copies = volumes * (copy_pitch(d->n) != d->n ? 2 : 1);
   const int64_t plain = std::min<int64_t>((int64_t)work_bytes / per_entry, entries);
-  const size_t tb = (size_t)copies * transposed_bytes(d);
+  const size_t tb = (size_t)copies * copy_bytes(d);
   const int64_t with_t = work_bytes > tb ? std::min<int64_t>((int64_t)(work_bytes - tb) / per_entry, entries) : 0;
   if (copies > 0 && with_t >= 1 && 2 * with_t >= plain) {
     *prefix = tb;
@@ -624,6 +688,12 @@ int64_t maps_bytes_per_angle(const cct_maps_desc* d) {
   return jobs * (P * P + P) * (int64_t)sizeof(float) * d->n_slices;  // W planes + partner constants
 }
 
+template <bool PAIRS>
+static void launch_scan(const MapsPass& p, int jobs, int slices, cudaStream_t st) {
+  (void)ensure_dynamic_smem<maps_scan_kernel<PAIRS>>((int)SCAN_SMEM);  // without it the launch fails and reports
+  maps_scan_kernel<PAIRS><<<dim3((p.P + SCAN_COLS - 1) / SCAN_COLS, jobs, slices), SCAN_THREADS, SCAN_SMEM, st>>>(p);
+}
+
 // Quarter-turn quads: per pass, the incident fields of 2 entries per quad (one job each, so a quad
 // takes the workspace of one entry with incident and emitted jobs), then one quad resample.
 static int launch_maps_quads(const cct_maps_desc* d, const float* mu_in, void* maps, void* work, size_t work_bytes,
@@ -636,11 +706,12 @@ static int launch_maps_quads(const cct_maps_desc* d, const float* mu_in, void* m
   if (per_pass < 1) return CCT_ERR_VALUE;
   per_pass = std::min(per_pass, 65535 / 2);
   MapsPass p;
-  p.mu_in_t = p.mu_out_t = nullptr;
+  p.mu_in_t = p.mu_out_t = p.mu_in_p = p.mu_out_p = nullptr;
+  p.pitch = copy_pitch(d->n);
   if (prefix > 0) {
-    p.mu_in_t = reinterpret_cast<float*>(work);
-    launch_transpose(mu_in, const_cast<float*>(p.mu_in_t), d->n, d->n_slices, st);
-    work = reinterpret_cast<char*>(work) + prefix;
+    char* w = reinterpret_cast<char*>(work);
+    launch_copies(d, mu_in, &w, &p.mu_in_t, &p.mu_in_p, st);
+    work = w;
   }
   p.n = d->n; p.P = P; p.e = e; p.n_det = 1; p.n_sub = 1;
   p.has_in = 1; p.has_out = 0; p.maps_dtype = d->maps_dtype; p.n_angles = d->n_angles;
@@ -654,7 +725,7 @@ static int launch_maps_quads(const cct_maps_desc* d, const float* mu_in, void* m
     const int nq = std::min(per_pass, d->n_quads - q0);
     p.a0 = q0;
     p.na = 2 * nq;
-    maps_scan_kernel<true><<<dim3((P + 127) / 128, p.na, d->n_slices), 128, 0, st>>>(p);
+    launch_scan<true>(p, p.na, d->n_slices, st);
     maps_resample_quad_kernel<<<dim3((unsigned)(tiles * tiles), nq, d->n_slices), 256, 0, st>>>(p);
   }
   return CCT_OK;
@@ -668,7 +739,7 @@ int launch_maps(const cct_maps_desc* d, const float* mu_in, const float* mu_out,
   const int entries = d->pairs != nullptr ? d->n_entries : d->n_angles;
   if (entries < 1 || entries > d->n_angles) return CCT_ERR_VALUE;
   if (d->quads != nullptr) return launch_maps_quads(d, mu_in, maps, work, work_bytes, st);
-  // transposed copies of mu_in and of a distinct mu_out
+  // copies of mu_in and of a distinct mu_out
   const bool out_own = d->has_out && (!d->has_in || mu_out != mu_in);
   const int copies = (d->has_in ? 1 : 0) + (out_own ? 1 : 0);
   size_t prefix = 0;
@@ -680,22 +751,18 @@ int launch_maps(const cct_maps_desc* d, const float* mu_in, const float* mu_out,
   per_pass = std::max(1, std::min(per_pass, 65535 / std::max(1, jobs)));
   if ((int64_t)jobs > 65535) return CCT_ERR_VALUE;
   MapsPass p;
-  p.mu_in_t = p.mu_out_t = nullptr;
+  p.mu_in_t = p.mu_out_t = p.mu_in_p = p.mu_out_p = nullptr;
+  p.pitch = copy_pitch(d->n);
   if (prefix > 0) {
-    float* t = reinterpret_cast<float*>(work);
-    const size_t tb = transposed_bytes(d);
-    if (d->has_in) {
-      launch_transpose(mu_in, t, d->n, d->n_slices, st);
-      p.mu_in_t = t;
-      t = reinterpret_cast<float*>(reinterpret_cast<char*>(t) + tb);
-    }
+    char* w = reinterpret_cast<char*>(work);
+    if (d->has_in) launch_copies(d, mu_in, &w, &p.mu_in_t, &p.mu_in_p, st);
     if (out_own) {
-      launch_transpose(mu_out, t, d->n, d->n_slices, st);
-      p.mu_out_t = t;
+      launch_copies(d, mu_out, &w, &p.mu_out_t, &p.mu_out_p, st);
     } else if (d->has_out) {
       p.mu_out_t = p.mu_in_t;
+      p.mu_out_p = p.mu_in_p;
     }
-    work = reinterpret_cast<char*>(work) + prefix;
+    work = w;
   }
   p.n = d->n; p.P = P; p.e = e; p.n_det = d->n_det; p.n_sub = d->n_sub;
   p.has_in = d->has_in; p.has_out = d->has_out; p.maps_dtype = d->maps_dtype; p.n_angles = d->n_angles;
@@ -707,11 +774,10 @@ int launch_maps(const cct_maps_desc* d, const float* mu_in, const float* mu_out,
   for (int a0 = 0; a0 < entries; a0 += per_pass) {
     p.a0 = a0;
     p.na = std::min(per_pass, entries - a0);
-    const dim3 g1((P + 127) / 128, p.na * p.jobs_per_angle, d->n_slices);
     if (p.pairs != nullptr) {
-      maps_scan_kernel<true><<<g1, 128, 0, st>>>(p);
+      launch_scan<true>(p, p.na * p.jobs_per_angle, d->n_slices, st);
     } else {
-      maps_scan_kernel<false><<<g1, 128, 0, st>>>(p);
+      launch_scan<false>(p, p.na * p.jobs_per_angle, d->n_slices, st);
     }
     const int tiles = (d->n + RS_TILE - 1) / RS_TILE;
     const dim3 g2((unsigned)(tiles * tiles), p.na, d->n_slices);
@@ -723,6 +789,15 @@ int launch_maps(const cct_maps_desc* d, const float* mu_in, const float* mu_out,
     }
   }
   return CCT_OK;
+}
+
+int read_scan_error(int clear, int* value) {
+  cudaError_t e = cudaMemcpyFromSymbol(value, g_scan_overflow, sizeof(int));
+  if (e == cudaSuccess && clear) {
+    const int zero = 0;
+    e = cudaMemcpyToSymbol(g_scan_overflow, &zero, sizeof(int));
+  }
+  return (int)e;
 }
 
 }  // namespace cct

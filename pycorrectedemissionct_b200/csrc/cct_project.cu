@@ -1519,6 +1519,8 @@ void launch_bp(const BpArgs& a, cudaStream_t st) {
 }  // namespace cct
 
 namespace cct {
+int read_scan_error(int clear, int* value);  // cct_maps.cu
+
 int read_device_error(int clear, int* value) {
   int v = 0;
   cudaError_t e = cudaMemcpyFromSymbol(&v, g_box_overflow, sizeof(int));
@@ -1533,7 +1535,10 @@ int read_device_error(int clear, int* value) {
     e = cudaMemcpyToSymbol(g_tma_timeout, &zero, sizeof(int));
     if (e != cudaSuccess) return (int)e;
   }
-  *value = v | (t << 1);
+  int m = 0;
+  const int rc = read_scan_error(clear, &m);
+  if (rc != 0) return rc;
+  *value = v | (t << 1) | (m << 2);
   return 0;
 }
 }  // namespace cct

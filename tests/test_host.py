@@ -666,3 +666,42 @@ def test_bp_edge_decision_equals_double(n):
         assert np.array_equal(np.where(left, d >= 0, d <= 0), (td >= -K) & (td <= n - 1 - K))
         checked += len(td)
     assert checked > 0
+
+
+@pytest.mark.parametrize("n,n_angles", [(2, 16), (3, 16), (33, 24), (130, 16), (251, 8), (512, 6)])
+def test_maps_scan_boxes_hold_every_tap(n, n_angles):
+    """The maps scan stages, per 64 columns x 64 support rows of a job, the bounding box of the samples
+    (scan_band in csrc/cct_maps.cu: at most 94 rows of 103 pixels) and reads the taps without tests;
+    mirror the FP32 box and positions and check every tap, for the incident and emitted rotations, and
+    that the band's rows contain the support rows of each of its columns."""
+    from pycorrectedemissionct_b200 import geometry
+
+    f = np.float32
+    e, P = geometry.padded_size(n)
+    angles = np.concatenate([np.linspace(0, 2 * np.pi, n_angles, endpoint=False), [np.pi / 4, 1e-7, 2.0]])
+    rot_in, rot_out, _ = geometry.attenuation_rotations(np.array(angles, dtype=f), [np.pi / 2], n)
+    for Md in [rot_in[a, 0] for a in range(len(angles))] + [rot_out[a, 0, 0, 0] for a in range(len(angles))]:
+        m00, m01, m02, m10, m11, m12 = f(Md[0]), f(Md[1]), f(Md[2] - e), f(Md[3]), f(Md[4]), f(Md[5] - e)
+        for tr in (False, True):
+            for c0 in range(0, P, 64):
+                cols = np.minimum(np.arange(c0, c0 + 64), P - 1)
+                sup = [_column_range(Md[0] * c + Md[2] - e, Md[1], Md[3] * c + Md[5] - e, Md[4], -1.0, float(n), P, True)
+                       for c in range(c0, min(c0 + 64, P))]
+                sup = [s for s in sup if s[0] <= s[1]]
+                if not sup:
+                    continue
+                blo, bhi = min(s[0] for s in sup), max(s[1] for s in sup)
+                xc, yc = _fma32(m00, cols.astype(f), m02), _fma32(m10, cols.astype(f), m12)
+                for r0 in range(blo, bhi + 1, 64):
+                    r1 = min(r0 + 63, bhi)
+                    cr = np.array([r0, r1], dtype=f)[:, None]
+                    ends = [0, min(c0 + 63, P - 1) - c0]
+                    bx, by = _fma32(m01, cr, xc[None, ends]), _fma32(m11, cr, yc[None, ends])
+                    (u, v) = (by, bx) if tr else (bx, by)
+                    bu, bu1 = (int(np.floor(u.min())) - 1) & ~3, int(np.floor(u.max())) + 2
+                    bv, bv1 = int(np.floor(v.min())) - 1, int(np.floor(v.max())) + 2
+                    assert bu1 - bu + 1 <= 103 and bv1 - bv + 1 <= 94
+                    rr = np.arange(r0, r1 + 1, dtype=f)[:, None]
+                    x, y = np.floor(_fma32(m01, rr, xc[None, :])), np.floor(_fma32(m11, rr, yc[None, :]))
+                    (u, v) = (y, x) if tr else (x, y)
+                    assert u.min() >= bu and u.max() + 1 <= bu1 and v.min() >= bv and v.max() + 1 <= bv1

@@ -1174,54 +1174,105 @@ __global__ void __launch_bounds__(BP_THREADS, 4) bp_ragged_kernel(const BpArgs* 
 // ------------------------------------------------------------------------------------------
 // Exact adjoint of the forward projection (gather form; no reference counterpart)
 // bp[p] = sum_a sum_{(r,c)} w_a hat(col_in(r,c) - p_x) hat(row_in(r,c) - p_y) y[a][c] (* map[a][p])
-// For a pixel p and angle a the candidate samples are the rotated-lattice points within
-// distance < 1 (per axis) of p: r, c within +-2 of the inverse-rotated position.
+// For a pixel p and angle a the samples that reach it lie within distance < 1 (per axis) of p, so within
+// sqrt(2) < 1.42 of its inverse-rotated lattice position along r and along c: at most three
+// values of each, ceil(position - 1.42) and the next two.
+//
+// Bound: issue (~110 instructions per pixel and line for the nine candidates).  A CTA holds 64 pixels
+// and four threads of each take every fourth line, since one thread per pixel leaves most of the
+// chip's warps empty at 256^2.  256^2 x 360: 1134 us with 36 candidates in FP64 per thread and
+// line, 211 us so.  The line sums and the sum over lines stay FP64.
 // ------------------------------------------------------------------------------------------
+constexpr int ADJ_PIXELS = 64;
+constexpr int ADJ_SPLIT = 4;
+constexpr int ADJ_CHUNK = 32;       // lines whose geometry is staged together
+constexpr float ADJ_REACH = 1.42f;  // > sqrt(2), by more than the FP32 error of the inverse position
+
+struct AdjLine {
+  float m00, m01, m02, m10, m11, m12;  // the forward map
+  float cx, cy, c0, rx, ry, r0;        // lattice column and row of a pixel: cx x + cy y + c0, ...
+  float w;
+  int angle, det;
+};
+
 template <bool HAS_MAPS, int MAPS_DTYPE>
-__global__ void __launch_bounds__(256) bp_adjoint_kernel(BpArgs args) {
+__global__ void __launch_bounds__(ADJ_PIXELS* ADJ_SPLIT) bp_adjoint_kernel(BpArgs args) {
+  __shared__ AdjLine lines[ADJ_CHUNK];
+  __shared__ double part[ADJ_SPLIT][ADJ_PIXELS];
   const int n = args.n;
   const int64_t total = (int64_t)n * n;
   const int s = blockIdx.y;
-  const int64_t pix = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix >= total) return;
-  const int pi = (int)(pix / n), pj = (int)(pix - (int64_t)pi * n);
+  const int tid = threadIdx.x, t = tid % ADJ_PIXELS, g = tid / ADJ_PIXELS;
+  const int64_t pix = (int64_t)blockIdx.x * ADJ_PIXELS + t;
+  const bool in = pix < total;
+  const int pi = in ? (int)(pix / n) : 0, pj = in ? (int)(pix - (int64_t)pi * n) : 0;
+  const float fi = (float)pi, fj = (float)pj;
   const int n_lines = args.n_det * args.n_angles;
   const float* sino = args.sino + (int64_t)s * n_lines * n;
   double acc = 0.0;
-  for (int l = 0; l < n_lines; ++l) {
-    const int d = l / args.n_angles;
-    const int a = l - d * args.n_angles;
-    const float* M = args.fp_matrix + 6 * a;
-    const float m00 = M[0], m01 = M[1], m02 = M[2], m10 = M[3], m11 = M[4], m12 = M[5];
-    // invert the 2x2 part to find the lattice point nearest to p
-    const double det = (double)m00 * m11 - (double)m01 * m10;
-    const double dx = pj - (double)m02, dy = pi - (double)m12;
-    const double cc = (m11 * dx - m01 * dy) / det;
-    const double rr = (-m10 * dx + m00 * dy) / det;
-    const int cb = (int)floor(cc), rb = (int)floor(rr);
-    double lsum = 0.0;
-    for (int r = rb - 2; r <= rb + 3; ++r) {
-      if (r < 0 || r >= n) continue;
-      for (int c = cb - 2; c <= cb + 3; ++c) {
-        if (c < 0 || c >= n) continue;
-        // same float arithmetic as the forward kernel's sample position
-        const float px = sample_x(m00, m01, m02, (float)c, (float)r);
-        const float py = sample_x(m10, m11, m12, (float)c, (float)r);
-        const float hx = 1.f - fabsf(px - (float)pj);
-        const float hy = 1.f - fabsf(py - (float)pi);
-        if (hx > 0.f && hy > 0.f) lsum += (double)hx * hy * sino[((int64_t)d * args.n_angles + a) * n + c];
+  for (int l0 = 0; l0 < n_lines; l0 += ADJ_CHUNK) {
+    const int count = min(ADJ_CHUNK, n_lines - l0);
+    __syncthreads();
+    if (tid < count) {
+      const int l = l0 + tid;
+      const int d = l / args.n_angles;
+      const int a = l - d * args.n_angles;
+      const float* M = args.fp_matrix + 6 * a;
+      AdjLine al;
+      al.m00 = M[0]; al.m01 = M[1]; al.m02 = M[2]; al.m10 = M[3]; al.m11 = M[4]; al.m12 = M[5];
+      const double det = (double)M[0] * M[4] - (double)M[1] * M[3];
+      al.cx = (float)(M[4] / det);
+      al.cy = (float)(-M[1] / det);
+      al.c0 = (float)(((double)M[1] * M[5] - (double)M[4] * M[2]) / det);
+      al.rx = (float)(-M[3] / det);
+      al.ry = (float)(M[0] / det);
+      al.r0 = (float)(((double)M[3] * M[2] - (double)M[0] * M[5]) / det);
+      al.w = args.weights != nullptr ? args.weights[a * args.n_det + d] : 1.f;
+      al.angle = a;
+      al.det = d;
+      lines[tid] = al;
+    }
+    __syncthreads();
+    for (int ll = g; in && ll < count; ll += ADJ_SPLIT) {
+      const AdjLine al = lines[ll];
+      const float cb = ceilf(fmaf(al.cx, fj, fmaf(al.cy, fi, al.c0)) - ADJ_REACH);
+      const float rb = ceilf(fmaf(al.rx, fj, fmaf(al.ry, fi, al.r0)) - ADJ_REACH);
+      const float* y = sino + (int64_t)(l0 + ll) * n;
+      // rows outside the lattice go far away, where the hat of the axis that r moves is zero
+      float2 fr[3];
+#pragma unroll
+      for (int dr = 0; dr < 3; ++dr) {
+        const float r = rb + (float)dr;
+        fr[dr].x = fr[dr].y = r >= 0.f && r <= (float)(n - 1) ? r : 1.0e9f;
       }
+      double lsum = 0.0;
+#pragma unroll
+      for (int dc = 0; dc < 3; ++dc) {
+        const float fc = cb + (float)dc;
+        const int c = (int)fc;
+        if ((unsigned)c >= (unsigned)n) continue;
+        const float2 pc = make_float2(fmaf(al.m00, fc, al.m02), fmaf(al.m10, fc, al.m12));
+        float h = 0.f;
+#pragma unroll
+        for (int dr = 0; dr < 3; ++dr) {
+          // same float arithmetic as the forward kernel's sample position (sample_x)
+          const float2 d = __fadd2_rn(__ffma2_rn(make_float2(al.m01, al.m11), fr[dr], pc), make_float2(-fj, -fi));
+          h = fmaf(fmaxf(1.f - fabsf(d.x), 0.f), fmaxf(1.f - fabsf(d.y), 0.f), h);
+        }
+        lsum += (double)h * (double)__ldg(y + c);
+      }
+      double contrib = lsum * al.w;
+      if (HAS_MAPS) {
+        const MapRef mr = make_map_ref(args.maps, MAPS_DTYPE, args.maps_slice_stride, args.n_angles, args.n_det, n, s,
+                                       al.angle, al.det, args.n_channels, args.chan_scale);
+        contrib *= map_at<MAPS_DTYPE>(mr, pix);
+      }
+      acc += contrib;
     }
-    float w = args.weights != nullptr ? args.weights[a * args.n_det + d] : 1.f;
-    double contrib = lsum * w;
-    if (HAS_MAPS) {
-      const MapRef mr = make_map_ref(args.maps, MAPS_DTYPE, args.maps_slice_stride, args.n_angles, args.n_det, n, s, a, d,
-                                     args.n_channels, args.chan_scale);
-      contrib *= map_at<MAPS_DTYPE>(mr, pix);
-    }
-    acc += contrib;
   }
-  bp_epilogue<BP_EPI_STORE>(args, s, pi, pj, (float)acc);
+  part[g][t] = acc;
+  __syncthreads();
+  if (g == 0 && in) bp_epilogue<BP_EPI_STORE>(args, s, pi, pj, (float)((part[0][t] + part[1][t]) + (part[2][t] + part[3][t])));
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1496,15 +1547,15 @@ void launch_bp_ragged(const BpArgs* groups, const int64_t* start, int n_groups, 
 
 void launch_bp(const BpArgs& a, cudaStream_t st) {
   if (a.mode == CCT_BP_ADJOINT) {
-    const dim3 grid((unsigned)(((int64_t)a.n * a.n + 255) / 256), a.n_slices);
+    const dim3 grid((unsigned)(((int64_t)a.n * a.n + ADJ_PIXELS - 1) / ADJ_PIXELS), a.n_slices);
     if (a.maps == nullptr) {
-      bp_adjoint_kernel<false, CCT_DTYPE_F32><<<grid, 256, 0, st>>>(a);
+      bp_adjoint_kernel<false, CCT_DTYPE_F32><<<grid, ADJ_PIXELS * ADJ_SPLIT, 0, st>>>(a);
     } else if (a.maps_dtype == CCT_DTYPE_BF16) {
-      bp_adjoint_kernel<true, CCT_DTYPE_BF16><<<grid, 256, 0, st>>>(a);
+      bp_adjoint_kernel<true, CCT_DTYPE_BF16><<<grid, ADJ_PIXELS * ADJ_SPLIT, 0, st>>>(a);
     } else if (a.maps_dtype == CCT_DTYPE_FIELDS_F32) {
-      bp_adjoint_kernel<true, CCT_DTYPE_FIELDS_F32><<<grid, 256, 0, st>>>(a);
+      bp_adjoint_kernel<true, CCT_DTYPE_FIELDS_F32><<<grid, ADJ_PIXELS * ADJ_SPLIT, 0, st>>>(a);
     } else {
-      bp_adjoint_kernel<true, CCT_DTYPE_F32><<<grid, 256, 0, st>>>(a);
+      bp_adjoint_kernel<true, CCT_DTYPE_F32><<<grid, ADJ_PIXELS * ADJ_SPLIT, 0, st>>>(a);
     }
     return;
   }

@@ -1,0 +1,36 @@
+"""GPU: the exact adjoint at the edges of its kernel (64 pixels per CTA, lines in chunks of 32, four threads
+per pixel) against the scatter definition in FP64, with and without maps, for odd sides and several
+detectors."""
+
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5  # FP32 sample positions against FP64
+
+
+@pytest.mark.parametrize("n,n_ang,n_det", [(2, 3, 1), (8, 1, 1), (9, 32, 1), (33, 33, 2), (64, 5, 1), (71, 65, 1)])
+def test_adjoint_matches_port(n, n_ang, n_det):
+    from oracle import port
+    from pycorrectedemissionct_b200 import core
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    dev = torch.device("cuda", 0)
+    rng = np.random.default_rng(n * n_ang)
+    angles = np.linspace(0, 2 * np.pi, n_ang, endpoint=False) + (0.0 if n_ang > 1 else 0.3)
+    c = core.XrfCore(n, angles, n_det=n_det, device=dev)
+    _, deg32 = port.backend_angles(angles)
+    y = rng.uniform(0.5, 1.5, size=(2, n_det, n_ang, n)).astype(np.float32)
+    maps = rng.uniform(0.3, 1.0, size=(2, n_ang, n_det, n, n)).astype(np.float32)
+    got = c.bp(torch.from_numpy(y).to(dev), "adjoint", torch.from_numpy(maps).to(dev)).double().cpu().numpy()
+    for s in range(2):
+        ref = port.fp_xrf_adjoint(y[s].astype(np.float64), maps[s].astype(np.float64), deg32, n)
+        assert rel_l2(got[s], ref) < TOL
+    if n_det == 1:
+        got = c.bp(torch.from_numpy(y).to(dev), "adjoint").double().cpu().numpy()
+        assert rel_l2(got[1], port.fp_xrf_adjoint(y[1, 0].astype(np.float64), None, deg32, n)) < TOL

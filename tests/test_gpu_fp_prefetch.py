@@ -1,0 +1,27 @@
+"""Forward projection with the next chunk's map rows asked for ahead: rows of any alignment and width."""
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,first", [(65, 1), (66, 0), (129, 1), (130, 3), (132, 1), (257, 2)])
+def test_fp_with_maps_at_odd_rows_equals_fp_of_the_product(n, first, dtype):
+    """One detector, unit weights: fp(x, map) of one angle is fp(x * map) of that angle, bit for bit (the
+    staged product is the same FP32 product), for sizes with a second chunk, rows that are not whole
+    16-byte units and maps that begin at any element of their buffer."""
+    from pycorrectedemissionct_b200 import core
+
+    a = 9
+    c = core.XrfCore(n, np.linspace(0.1, 2 * np.pi, a))
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.rand((1, n, n), device="cuda", generator=g)
+    buf = (torch.rand(first + a * n * n, device="cuda", generator=g) + 0.5).to(dtype)
+    maps = buf[first:].view(1, a, 1, n, n)
+    sino = c.fp(x, maps)
+    for k in range(a):
+        one = core.XrfCore(n, np.linspace(0.1, 2 * np.pi, a)[k : k + 1])
+        assert torch.equal(sino[:, :, k], one.fp(x * maps[:, k, 0].float())[:, :, 0])

@@ -210,6 +210,9 @@ __device__ __forceinline__ void fp_cta(const FpArgs& args, const int band, const
   const float fc = (float)c;
   const float pxc = fmaf(m00, fc, m02);
   const float pyc = fmaf(m10, fc, m12);
+  constexpr bool SKIP = HAS_MAPS && MAPS_DTYPE == CCT_DTYPE_FIELDS_F32;
+  const float idet = SKIP ? 1.f / (m00 * m11 - m01 * m10) : 0.f;  // inverse of the rotation part
+  const float i00 = m11 * idet, i01 = -m01 * idet, i10 = -m10 * idet, i11 = m00 * idet;
 
   // thread t computes the box of row chunk t (n <= 8192: at most FP_MAX_CHUNKS chunks)
   if (tid * FP_TR < n) {
@@ -235,6 +238,16 @@ __device__ __forceinline__ void fp_cta(const FpArgs& args, const int band, const
     if (HAS_MAPS && MAPS_DTYPE != CCT_DTYPE_FIELDS_F32 && r0 + FP_TR < n) fp_prefetch_rows<MAPS_DTYPE>(mref, n, box_sh[r0 / FP_TR + 1], tid);
     // Stage z = vol * map over the box (zeros outside the image); every thread takes items
     // tid, tid + 256, ... of the q4 x bh grid, issuing FP_FILL_BATCH items' loads at once.
+    // Line-integral fields pay four expf per quad, so quads that no tap reads are left out: a tap of
+    // a sample at (c, r) lies in the quad (columns gx .. gx + 3 of row gy) only if the sample's
+    // position is within (2.5, 1) of (gx + 1.5, gy); taken back to lattice coordinates, the quad is
+    // needed only if |c - cm| <= hc and |r - rm| <= hr (0.05 for rounding).  About half of a box's
+    // quads fail at 45 degrees.  PDHG 1024x720, 4 channels: 9.39 -> 9.10 ms an iteration; with stored
+    // maps the test costs more than the loads it saves (MLEM 512x720 15.8 -> 16.9 ms).
+    const float cm = 0.5f * (float)(c0 + c_last), rm = 0.5f * (float)(r0 + r_last);
+    const float qc0 = fmaf(i00, 1.5f - m02, -i01 * m12) - cm, qr0 = fmaf(i10, 1.5f - m02, -i11 * m12) - rm;
+    const float hc = 0.5f * (float)(c_last - c0) + 2.5f * fabsf(i00) + fabsf(i01) + 0.05f;
+    const float hr = 0.5f * (float)(r_last - r0) + 2.5f * fabsf(i10) + fabsf(i11) + 0.05f;
     const int items = q4 * bh;
     // it / q4 = (it * ceil(2^20 / q4)) >> 20, exact for it < 2^12 and q4 <= 25 (the error
     // it * (magic - 2^20 / q4) / 2^20 < 2^-8 stays below 1 / q4), and the product fits 32 bits
@@ -251,6 +264,11 @@ __device__ __forceinline__ void fp_cta(const FpArgs& args, const int band, const
           const int rr = (int)(((unsigned)it * magic) >> 20);
           const int qq = it - rr * q4;
           const int gy = by0 + rr, gx = bx0 + 4 * qq;
+          if (SKIP) {
+            const float fy = (float)gy, fx = (float)gx;
+            const float qc = fmaf(i00, fx, fmaf(i01, fy, qc0)), qr = fmaf(i10, fx, fmaf(i11, fy, qr0));
+            if (fabsf(qc) > hc || fabsf(qr) > hr) continue;
+          }
           dst[k] = rr * FP_STRIDE + 4 * qq;
           if (vec4) {
             // n % 4 == 0 and gx % 4 == 0: a float4 is either fully inside or fully outside

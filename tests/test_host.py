@@ -705,3 +705,34 @@ def test_maps_scan_boxes_hold_every_tap(n, n_angles):
                     x, y = np.floor(_fma32(m01, rr, xc[None, :])), np.floor(_fma32(m11, rr, yc[None, :]))
                     (u, v) = (y, x) if tr else (x, y)
                     assert u.min() >= bu and u.max() + 1 <= bu1 and v.min() >= bv and v.max() + 1 <= bv1
+
+
+@pytest.mark.parametrize("n,n_angles", [(2, 8), (65, 24), (131, 16), (512, 12), (8192, 12)])
+def test_fp_fields_fill_keeps_every_tap_quad(n, n_angles):
+    """With line-integral fields the forward projection leaves out quads of a chunk's box that no tap
+    reads (fp_cta in csrc/cct_project.cu); mirror the FP32 test over chunks of 64 columns x 64 rows."""
+    from pycorrectedemissionct_b200 import geometry
+
+    f = np.float32
+    angles = np.concatenate([np.linspace(0, 360, n_angles, endpoint=False), [45.0, 1e-5, 89.99999]])
+    rng = np.random.default_rng(n)
+    chunks = [(c, r) for c in range(0, n, 64) for r in range(0, n, 64)]
+    corners = [chunks[0], chunks[-1], chunks[len(chunks) // 2]]
+    for m in geometry.fp_matrices(angles.astype(f), n).reshape(-1, 6).astype(f):
+        m00, m01, m02, m10, m11, m12 = m
+        idet = f(1) / (m00 * m11 - m01 * m10)
+        i00, i01, i10, i11 = m11 * idet, -m01 * idet, -m10 * idet, m00 * idet
+        for c0, r0 in corners + [chunks[k] for k in rng.integers(0, len(chunks), 4)]:
+            c1, r1 = min(c0 + 64, n) - 1, min(r0 + 64, n) - 1
+            c, r = np.arange(c0, c1 + 1, dtype=f)[None, :], np.arange(r0, r1 + 1, dtype=f)[:, None]
+            x = np.floor(_fma32(m01, r, _fma32(m00, c, m02)))
+            y = np.floor(_fma32(m11, r, _fma32(m10, c, m12)))
+            cm, rm = f(0.5) * f(c0 + c1), f(0.5) * f(r0 + r1)
+            qc0 = _fma32(i00, f(1.5) - m02, -i01 * m12) - cm
+            qr0 = _fma32(i10, f(1.5) - m02, -i11 * m12) - rm
+            hc = f(0.5) * f(c1 - c0) + f(2.5) * abs(i00) + abs(i01) + f(0.05)
+            hr = f(0.5) * f(r1 - r0) + f(2.5) * abs(i10) + abs(i11) + f(0.05)
+            for dx, dy in ((0, 0), (1, 0), (0, 1), (1, 1)):
+                gx, gy = (np.floor((x + dx) / 4) * 4).astype(f), (y + dy).astype(f)
+                assert abs(_fma32(i00, gx, _fma32(i01, gy, qc0))).max() <= hc
+                assert abs(_fma32(i10, gx, _fma32(i11, gy, qr0))).max() <= hr

@@ -53,6 +53,7 @@ struct ConvArgs {
   __nv_bfloat16* y;    // NHWC output
   int relu, wide;      // wide: y is 32-byte aligned
   int stages, resident;
+  int whole;           // a stage holds the three boxes of a tile (one channel block, weights resident)
 };
 
 struct WgradArgs {
@@ -181,11 +182,13 @@ __host__ __device__ inline uint32_t net_tmem_cols(int cols) {
 // write the results of the tile before from the other TMEM accumulator (a pair of warps per quarter
 // of its lanes, each with half of the columns: with one warp per quarter and integer divisions
 // for the tile's place, that chain of ~500 dependent instructions was what a tile took).  A tile is 8 columns x 16
-// (or, in pairs that share the weights, 32) rows of output pixels, one TMEM lane each.  For a
-// horizontal tap dx and a block of input channels, one TMA box of 8 x (rows + 2) pixels, zero
-// outside the image, serves the three vertical taps: 8 pixels of a row are one swizzle atom, so a
-// tap is the box from dy rows on.  Weights stay in shared memory for all tiles of a CTA where
-// they fit beside the pixel boxes, and are loaded with each box otherwise.
+// (or, in pairs that share the weights, 32) rows of output pixels, one TMEM lane each.  The sum runs
+// over taps in row order, then channels: TMEM rounds by truncation, so another order moves the
+// results, and 15 layers of BF16 rounding make 0.5 % of such a difference (dx outermost: 1.19 ms for the
+// network instead of 1.21 ms).  Up to 64 x 64 channels the weights stay in shared memory and a
+// stage is a tile's three boxes of 8 x 18 pixels, one per horizontal tap, zero outside the image:
+// 8 pixels of a row are one swizzle atom, so a vertical tap is a box from dy rows on.  With more
+// channels a stage is one tap: its box of pixels and, unless they stay, its weights.
 // ----------------------------------------------------------------------------------------------
 constexpr int CONV_THREADS = 320;
 
@@ -216,10 +219,12 @@ __global__ void __launch_bounds__(CONV_THREADS)
   const int chunks = a.cin / ck;
   const int bn = a.cout < 128 ? a.cout : 128;
   const uint32_t cols = net_tmem_cols(2 * MT * bn);
-  const uint32_t x_bytes = (uint32_t)(NET_TW * (MT * NET_TH + 2) * ck * 2);
+  const bool whole = a.whole != 0;
+  const uint32_t x_bytes = (uint32_t)(NET_TW * (MT * NET_TH + (whole ? 2 : 0)) * ck * 2);
   const uint32_t w_bytes = (uint32_t)(bn * ck * 2);  // one tap
   const uint32_t x_pitch = (x_bytes + 1023) & ~1023u;
-  const uint32_t stage_bytes = x_pitch + (a.resident ? 0u : 3u * w_bytes);
+  const uint32_t stage_bytes = whole ? 3u * x_pitch : x_pitch + (a.resident ? 0u : w_bytes);
+  const int steps = whole ? 1 : 9 * chunks;  // stages of a tile
   const uint32_t w_base = 0, ring = a.resident ? 9u * chunks * w_bytes : 0u;
   const int items = a.tiles * a.n_tiles;
 
@@ -257,17 +262,22 @@ __global__ void __launch_bounds__(CONV_THREADS)
     bool ok = true;
     for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
       const ConvItem i = conv_item(a, it);
-      for (int dx = 0, c = 0; dx < 3; c + 1 == chunks ? (c = 0, ++dx) : ++c) {
+      for (int q = 0, t = 0, c = 0; q < steps; ++q, c + 1 == chunks ? (c = 0, ++t) : ++c) {
         if (sent >= a.stages && !net_mbar_wait(&empty[s], phase ^ 1u, abort)) {
           ok = false;
           break;
         }
         unsigned char* st = net_smem + ring + (uint32_t)s * stage_bytes;
-        net_mbar_expect(&full[s], x_bytes + (a.resident ? 0u : 3u * w_bytes));
-        tma_4d(st, &tm_x, c * ck, i.tx * NET_TW + dx - 1, i.ty * MT * NET_TH - 1, i.b, &full[s]);
-        if (!a.resident)
-          for (int dy = 0; dy < 3; ++dy)
-            tma_3d(st + x_pitch + (uint32_t)dy * w_bytes, &tm_w, c * ck, 3 * dy + dx, i.nt * bn, &full[s]);
+        if (whole) {
+          net_mbar_expect(&full[s], 3u * x_bytes);
+          for (int dx = 0; dx < 3; ++dx)
+            tma_4d(st + (uint32_t)dx * x_pitch, &tm_x, 0, i.tx * NET_TW + dx - 1, i.ty * MT * NET_TH - 1, i.b, &full[s]);
+        } else {
+          const int dy = t / 3;
+          net_mbar_expect(&full[s], x_bytes + (a.resident ? 0u : w_bytes));
+          tma_4d(st, &tm_x, c * ck, i.tx * NET_TW + t - 3 * dy - 1, i.ty * MT * NET_TH + dy - 1, i.b, &full[s]);
+          if (!a.resident) tma_3d(st + x_pitch, &tm_w, c * ck, t, i.nt * bn, &full[s]);
+        }
         ++sent;
         if (++s == a.stages) {
           s = 0;
@@ -294,7 +304,7 @@ __global__ void __launch_bounds__(CONV_THREADS)
       const int buf = done & 1;
       if (done >= 2 && !net_mbar_wait(&acc_empty[buf], (uint32_t)(((done >> 1) & 1) ^ 1), abort)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      for (int q = 0, dx = 0, c = 0; q < 3 * chunks; ++q) {
+      for (int q = 0, t = 0, c = 0; q < steps; ++q) {
         if (!net_mbar_wait(&full[s], phase, abort)) {
           ok = false;
           break;
@@ -302,25 +312,37 @@ __global__ void __launch_bounds__(CONV_THREADS)
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t st = base + ring + (uint32_t)s * stage_bytes;
         const uint32_t xa = umma_desc_lo(st, 16);
-        const uint32_t wb = umma_desc_lo(a.resident ? base + w_base + (uint32_t)(c * 9 + dx) * w_bytes : st + x_pitch, 16);
-        const uint32_t w_step = (a.resident ? 3u * w_bytes : w_bytes) >> 4;
         const uint32_t acc = tmem + (uint32_t)(buf * MT * bn);
+        if (whole) {
+          const uint32_t wb = umma_desc_lo(base + w_base, 16), w_step = w_bytes >> 4, x_step = x_pitch >> 4;
 #pragma unroll
-        for (int dy = 0; dy < 3; ++dy) {
+          for (int tap = 0; tap < 9; ++tap) {
+#pragma unroll
+            for (int k = 0; k < CK / 16; ++k) {
+              const uint64_t bd = umma_desc(wb + tap * w_step + 2u * k, hi);
+#pragma unroll
+              for (int m = 0; m < MT; ++m)
+                umma_bf16(acc + (uint32_t)(m * bn),
+                          umma_desc(xa + (tap % 3) * x_step + (uint32_t)((m * NET_TH + tap / 3) * NET_TW * CK / 8) + 2u * k, hi),
+                          bd, idesc, tap > 0 || k > 0);
+            }
+          }
+        } else {
+          const uint32_t wb = umma_desc_lo(a.resident ? base + w_base + (uint32_t)(c * 9 + t) * w_bytes : st + x_pitch, 16);
 #pragma unroll
           for (int k = 0; k < CK / 16; ++k) {
-            const uint64_t bd = umma_desc(wb + dy * w_step + 2u * k, hi);
+            const uint64_t bd = umma_desc(wb + 2u * k, hi);
 #pragma unroll
             for (int m = 0; m < MT; ++m)
-              umma_bf16(acc + (uint32_t)(m * bn), umma_desc(xa + (uint32_t)((m * NET_TH + dy) * NET_TW * CK / 8) + 2u * k, hi), bd,
-                        idesc, q > 0 || dy > 0 || k > 0);
+              umma_bf16(acc + (uint32_t)(m * bn), umma_desc(xa + (uint32_t)(m * NET_TH * NET_TW * CK / 8) + 2u * k, hi), bd, idesc,
+                        q > 0 || k > 0);
           }
         }
         umma_commit(&empty[s]);
         ++issued;
         if (++c == chunks) {
           c = 0;
-          ++dx;
+          ++t;
         }
         if (++s == a.stages) {
           s = 0;
@@ -623,19 +645,21 @@ static int launch_conv_fwd(ConvArgs a, const void* x, const void* wt, cudaStream
   a.by_n = FastDiv(a.n_tiles);
   a.by_x = FastDiv(a.tiles_x);
   a.by_y = FastDiv(a.tiles_y);
-  const int x_pitch = (NET_TW * (MT * NET_TH + 2) * a.ck * 2 + 1023) / 1024 * 1024, w_tap = bn * a.ck * 2;
+  a.whole = a.resident && chunks == 1;
+  const int box_rows = MT * NET_TH + (a.whole ? 2 : 0);
+  const int x_pitch = (NET_TW * box_rows * a.ck * 2 + 1023) / 1024 * 1024, w_tap = bn * a.ck * 2;
   const int weights = 9 * chunks * w_tap;
-  const int stage = x_pitch + (a.resident ? 0 : 3 * w_tap);
+  const int stage = a.whole ? 3 * x_pitch : x_pitch + (a.resident ? 0 : w_tap);
   const int fixed = a.resident ? weights : 0;
   // two CTAs per SM where each still gets three stages, else as many stages as one CTA can hold
   const int half = 110 * 1024;
-  const int per_sm = fixed + 3 * stage <= half && 2 * net_tmem_cols(2 * MT * bn) <= 512 ? 2 : 1;
+  const int per_sm = fixed + (a.whole ? 2 : 3) * stage <= half && 2 * net_tmem_cols(2 * MT * bn) <= 512 ? 2 : 1;
   const int room = (per_sm == 2 ? half : NET_SMEM_MAX - 1024) - fixed;
   a.stages = std::min(8, room / stage);
   if (a.stages < 2) return net_fail("the convolution's operands do not fit in shared memory");
   const int smem = fixed + a.stages * stage + 1024;
   CUtensorMap tm_x, tm_w;
-  if (!net_map_nhwc(&tm_x, x, a.batch, a.h, a.w, a.cin, a.ck, MT * NET_TH + 2) ||
+  if (!net_map_nhwc(&tm_x, x, a.batch, a.h, a.w, a.cin, a.ck, box_rows) ||
       !net_map_weights(&tm_w, wt, a.cin, a.cout, a.ck, bn))
     return net_fail("cuTensorMapEncodeTiled refused the convolution's operands");
   if (!ensure_dynamic_smem<conv_fwd_kernel<MT, CK>>(NET_SMEM_MAX))

@@ -99,3 +99,10 @@ def test_elementwise_wide_and_narrow(c, offset):
     assert torch.equal(large.double(), rep / 4) and torch.equal(up.double(), rep)
     assert torch.equal(total.double(), x.double() + x2.double())
     assert torch.equal(db.double(), x.double().sum((0, 1, 2)))
+
+
+@pytest.mark.parametrize("b,h,w,cin,cout", [(1, 18, 11, 128, 32), (2, 16, 8, 256, 16), (1, 33, 9, 512, 16), (1, 7, 9, 64, 128)])
+def test_convolutions_of_one_tap_per_stage(b, h, w, cin, cout):
+    """Several channel blocks with weights that stay in shared memory (9 cin cout values in 74 KB at most) and
+    one block with weights that do not: both walk the taps one by one."""
+    test_convolutions_at_tile_edges(b, h, w, cin, cout)

@@ -157,22 +157,32 @@ __device__ __forceinline__ void fp_write_partial(double v, double* partials, int
   }
 }
 
-// Asks L2 for the FP32 map rows of a chunk's box, one bulk prefetch per row (whole 16-byte units inside
-// the row only).  The fill is bound by the latency of its loads (the long scoreboard is half of all
-// stalls): issued one chunk ahead, its map loads wait for L2 and not for HBM.  MLEM at 512x720, 16
-// slices: 8.4 -> 7.9 ms an iteration; 8 slices in subsets 7.43 -> 7.03 ms.  Asking after the fill
-// (2% slower) or two chunks ahead (no difference) gains less.  BF16 rows, half as long, are not asked for:
-// 1.61 -> 1.65 ms for 4 slices of 512x720 (FP32 1024x180, 2 slices: 0.95 -> 0.89 ms).  Line-integral
-// fields neither: their planes are shared by the channels' CTAs, which already find them in L2 (9.4 ->
-// 10.2 ms a 1024x720 4-channel iteration with every channel asking, 9.7 ms with one).
+// Asks L2 for the map rows of a chunk's box, a 128-byte line per request (the first at the row's start in
+// the box, so that every address lies inside the row).  The fill is bound by the latency of its loads
+// (the long scoreboard is half of all stalls): issued one chunk ahead, its map loads wait for L2 and not
+// for HBM.  MLEM at 512x720, 16 slices: 8.4 -> 7.6 ms an iteration, 8 slices in subsets 7.43 -> 6.70 ms,
+// 32 slices with BF16 maps 12.7 -> 11.8 ms a projection.  One bulk request per row
+// (cp.async.bulk.prefetch) does the same with more instructions, as its operands are uniform and
+// the lanes take turns: 7.9 ms, 6.98 ms and 13.0 ms.  Asking after the fill (2% slower) or two chunks
+// ahead (no difference) gains less.  Line-integral fields are not asked for: their planes are shared
+// by the channels' CTAs, which already find them in L2 (9.4 -> 10.2 ms a 1024x720 4-channel
+// iteration with every channel asking, 9.7 ms with one, both in bulk).
+template <int DT>
 __device__ __forceinline__ void fp_prefetch_rows(const MapRef& m, int n, const int4 box, int tid) {
-  const int y = box.z + tid;
-  if (y > box.w || (unsigned)y >= (unsigned)n) return;
+  constexpr int ES = DT == CCT_DTYPE_BF16 ? 2 : 4;
+  constexpr int LINES = DT == CCT_DTYPE_BF16 ? 2 : 4;  // lines of a row (of at most 400 bytes and where it begins in its first line)
   const int x0 = max(box.x, 0), x1 = min(box.y + 1, n);
-  if (x0 >= x1) return;
-  const uint64_t row = reinterpret_cast<uint64_t>(reinterpret_cast<const float*>(m.base) + m.off + (int64_t)y * n);
-  const uint64_t b = (row + 4 * (uint64_t)x0 + 15) & ~15ull, e = (row + 4 * (uint64_t)x1) & ~15ull;
-  if (b < e) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b), "r"((uint32_t)(e - b)) : "memory");
+  const int line = tid % LINES;
+#pragma unroll
+  for (int k = 0; k < (FP_BOX_H * LINES + FP_THREADS - 1) / FP_THREADS; ++k) {
+    const int y = box.z + tid / LINES + k * (FP_THREADS / LINES);
+    if (y > box.w || (unsigned)y >= (unsigned)n) continue;
+    const uint64_t row = reinterpret_cast<uint64_t>(m.base) + (uint64_t)(m.off + (int64_t)y * n) * ES;
+    const uint64_t b = row + (uint64_t)(x0 * ES), e = row + (uint64_t)(x1 * ES);
+    uint64_t at = (b & ~127ull) + 128ull * line;
+    if (line == 0) at = b;
+    if (at < e && x0 < x1) asm volatile("prefetch.global.L2 [%0];" ::"l"(at) : "memory");
+  }
 }
 
 // One CTA of the forward projection: detector band `band` of (angle, detector) `ad` of slice
@@ -237,7 +247,7 @@ __device__ __forceinline__ void fp_cta(const FpArgs& args, const int band, const
       return;
     }
 
-    if (HAS_MAPS && MAPS_DTYPE == CCT_DTYPE_F32 && r0 + FP_TR < n) fp_prefetch_rows(mref, n, box_sh[r0 / FP_TR + 1], tid);
+    if (HAS_MAPS && MAPS_DTYPE != CCT_DTYPE_FIELDS_F32 && r0 + FP_TR < n) fp_prefetch_rows<MAPS_DTYPE>(mref, n, box_sh[r0 / FP_TR + 1], tid);
     // Stage z = vol * map over the box (zeros outside the image); every thread takes items
     // tid, tid + 256, ... of the q4 x bh grid, issuing FILL_BATCH items' loads at once.
     // Line-integral fields pay four expf per quad, so quads that no tap reads are left out: a tap of

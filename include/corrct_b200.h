@@ -99,7 +99,9 @@ int cct_abi_version(void);
 const char* cct_last_error(void);
 
 /* Kernels never trap: an internal bound that valid inputs cannot exceed raises a device flag
-   instead.  *value = the flag (0 = clean); clear != 0 resets it.  Synchronous. */
+   instead.  *value = the flags (0 = clean; 1: a box of the forward projection
+   was too large, 2: a wait of its TMA variant ran out, 4: a box of the maps scan was too large);
+   clear != 0 resets them.  Synchronous. */
 int cct_device_error(int32_t clear, int32_t* value);
 
 /*

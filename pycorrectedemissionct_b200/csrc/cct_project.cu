@@ -909,9 +909,12 @@ struct BpShared {
 // double, where both products are exact; here the distance d past the edge is formed from the
 // products' FP32 halves, the exact error of their difference and a difference with the edge that
 // is exact too (Sterbenz), so that only the last sum rounds: at |d| < 0.02 by less than 1e-11, with the
-// sign of a d that is exactly 0 (angles of 0 and 90 degrees) intact.  bins points at the staged
-// pair of bin 0.
-__device__ __forceinline__ float bp_edge_value(const float2* bins, float cs, float sn, int n, float jc, float ic) {
+// sign of a d that is exactly 0 (angles of 0 and 90 degrees) intact.  A pixel on the edge itself takes the
+// edge bin as it is, like np.interp: the pair of bins n - 2 and n - 1 gives the latter only to the
+// rounding of their difference (0 for 3e7 and 0.5).  bins points at the staged pair of bin 0, line at the
+// unstaged bins and w is their weight.
+__device__ __forceinline__ float bp_edge_value(const float2* bins, const float* line, float w, float cs, float sn, int n,
+                                               float jc, float ic) {
   const int K = n / 2;
   const float p = jc * cs, pe = fmaf(jc, cs, -p);
   const float q = -ic * sn, qe = fmaf(-ic, sn, -q);
@@ -920,7 +923,9 @@ __device__ __forceinline__ float bp_edge_value(const float2* bins, float cs, flo
   const bool left = s < -0.5f;
   const float d = (s + (left ? (float)K : -(float)(n - 1 - K))) + (se + (pe + qe));
   if (left ? d < 0.f : d > 0.f) return 0.f;
+  if (!left && d == 0.f) return w * __ldg(line + (n - 1));
   const float2 v = bins[left ? 0 : n - 2];
+  if (d == 0.f) return v.x;
   return fmaf(left ? d : 1.f + d, v.y, v.x);
 }
 
@@ -1109,7 +1114,8 @@ __device__ __forceinline__ void bp_segment(const BpArgs& args, BpShared& sh, int
       for (int k = 0; k < PPT; ++k) {
         const float u = fmaf(k & 1 ? nfi[k / 2].y : nfi[k / 2].x, li.sn, base);
         if (fabsf(fabsf(u - li.mid) - li.half) >= BP_EDGE_GUARD) continue;
-        float v = bp_edge_value(pairs[ll] - li.kbase, li.cs, li.sn, n, fj, -(k & 1 ? nfi[k / 2].y : nfi[k / 2].x));
+        float v = bp_edge_value(pairs[ll] - li.kbase, sino + (int64_t)(lc + ll) * n, li.w, li.cs, li.sn, n, fj,
+                                -(k & 1 ? nfi[k / 2].y : nfi[k / 2].x));
         if (SYM) {
           const int l = lc + ll;
           const int d = l / args.n_angles;

@@ -41,3 +41,31 @@ def test_bp_matches_port_and_batches_agree(n, n_ang, n_det):
     es = rel_l2(sym[0].cpu().numpy(), port.bp_xrf(y64, m64, deg32, is_symmetric=True))
     report(f"bp n={n} lines={n_ang * n_det}", e, TOL)
     assert e < TOL and es < TOL
+
+
+@pytest.mark.parametrize("n_ang", [1, 16, 70])
+@pytest.mark.parametrize("n", [2, 3, 33, 64, 193])
+def test_bp_takes_the_last_bin_itself(n, n_ang):
+    """Lines at angle 0, whose last image column lies exactly on the last detector bin: np.interp returns that
+    bin, whatever its neighbour holds (3e7 beside 0.5 here, or infinity).  Every pixel is exactly on a bin
+    and every sum is exact in FP32, so the results are equal, for a batch on either side of the
+    cluster rule, in the reference and the symmetric mode."""
+    from pycorrectedemissionct_b200 import core
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    dev = torch.device("cuda", 0)
+    s = 352 // max(1, -(-n // 32) * -(-n // (64 if n > 192 else 32))) + 1
+    y = np.ones((1, n_ang, n), dtype=np.float32)
+    y[..., -2], y[..., -1] = 3e7, 0.5
+    c = core.XrfCore(n, np.zeros(n_ang), device=dev)
+    maps = torch.ones((s, n_ang, 1, n, n), device=dev)
+    t = np.arange(n) - n // 2
+    ref = n_ang * np.interp(t, t, y[0, 0].astype(np.float64), left=0, right=0)
+    yd = torch.from_numpy(y).to(dev).expand(s, -1, -1, -1).contiguous()
+    for slices in (1, s):
+        for args in (("reference",), ("symmetric", maps[:slices])):
+            got = c.bp(yd[:slices], *args).double().cpu().numpy()
+            assert np.array_equal(got, np.broadcast_to(ref, got.shape))
+    yd[..., -2] = float("inf")
+    assert torch.equal(c.bp(yd)[..., -1], torch.full((s, n), 0.5 * n_ang, device=dev))

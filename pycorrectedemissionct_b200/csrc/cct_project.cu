@@ -908,8 +908,9 @@ struct BpShared {
 // is within BP_EDGE_GUARD of a detector edge.  numpy decides the edge on t = jc cos - ic sin in
 // double, where both products are exact; here the distance d past the edge is formed from the
 // products' FP32 halves, the exact error of their difference and a difference with the edge that
-// is exact too (Sterbenz), so that only the last sum rounds: at |d| < 0.02 by less than 1e-11, with the
-// sign of a d that is exactly 0 (angles of 0 and 90 degrees) intact.  A pixel on the edge itself takes the
+// is exact too (Sterbenz), so that only the sum of the errors rounds: at |d| < 0.02 by less than 1e-11, with
+// the sign of a d that is exactly 0 (angles of 0 and 90 degrees) intact.  The value is interpolated in
+// FP64.  A pixel on the edge itself takes the
 // edge bin as it is, like np.interp: the pair of bins n - 2 and n - 1 gives the latter only to the
 // rounding of their difference (0 for 3e7 and 0.5).  bins points at the staged pair of bin 0, line at the
 // unstaged bins and w is their weight.
@@ -921,12 +922,12 @@ __device__ __forceinline__ float bp_edge_value(const float2* bins, const float* 
   const float s = p + q, b = s - p;
   const float se = (p - (s - b)) + (q - b);  // p + q = s + se exactly
   const bool left = s < -0.5f;
-  const float d = (s + (left ? (float)K : -(float)(n - 1 - K))) + (se + (pe + qe));
-  if (left ? d < 0.f : d > 0.f) return 0.f;
-  if (!left && d == 0.f) return w * __ldg(line + (n - 1));
+  const double d = (double)(s + (left ? (float)K : -(float)(n - 1 - K))) + (double)(se + (pe + qe));
+  if (left ? d < 0.0 : d > 0.0) return 0.f;
+  if (!left && d == 0.0) return w * __ldg(line + (n - 1));
   const float2 v = bins[left ? 0 : n - 2];
-  if (d == 0.f) return v.x;
-  return fmaf(left ? d : 1.f + d, v.y, v.x);
+  if (d == 0.0) return v.x;
+  return (float)fma(left ? d : 1.0 + d, (double)v.y, (double)v.x);
 }
 
 // Values of a staged line at two positions (bins from kbase), in packed FP32x2 arithmetic that rounds

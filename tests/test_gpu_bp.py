@@ -69,3 +69,29 @@ def test_bp_takes_the_last_bin_itself(n, n_ang):
             assert np.array_equal(got, np.broadcast_to(ref, got.shape))
     yd[..., -2] = float("inf")
     assert torch.equal(c.bp(yd)[..., -1], torch.full((s, n), 0.5 * n_ang, device=dev))
+
+
+@pytest.mark.parametrize("n", [33, 130, 251])
+def test_bp_interpolates_edge_pixels_in_double(n):
+    """Pixels within 0.01 bin inside the last detector bin, on a line that rises from -1 to 0 there: the value is
+    the distance to the edge itself, known to 1e-11 and rounded to FP32 once (formed in FP32 as
+    -1 + (1 + d) it would be off by up to 6e-8)."""
+    from oracle import port
+    from pycorrectedemissionct_b200 import core
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    dev = torch.device("cuda", 0)
+    y = np.zeros((1, 1, 1, n), dtype=np.float32)
+    y[..., -2] = -1.0
+    jj, ii = np.meshgrid(np.arange(n) - n // 2, np.arange(n) - n // 2)
+    checked = 0
+    for angle in np.random.default_rng(n).uniform(0, 2 * np.pi, 60):
+        _, deg32 = port.backend_angles(np.array([angle]))
+        rad = np.deg2rad(deg32[0])
+        d = (n - 1 - n // 2) - (jj * np.cos(rad).astype(np.float64) - ii * np.sin(rad).astype(np.float64))
+        near = (d > 0) & (d < 0.009)
+        got = core.XrfCore(n, [angle], device=dev).bp(torch.from_numpy(y).to(dev))[0].double().cpu().numpy()
+        assert np.all(np.abs(got + d)[near] <= 1e-11 + 2.0**-24 * d[near])
+        checked += int(near.sum())
+    assert checked > 0

@@ -1308,6 +1308,7 @@ __global__ void __launch_bounds__(ADJ_PIXELS* ADJ_SPLIT) bp_adjoint_kernel(BpArg
         const float fc = cb + (float)dc;
         const int c = (int)fc;
         if ((unsigned)c >= (unsigned)n) continue;
+        const float yc = __ldg(y + c);
         const float2 pc = make_float2(fmaf(al.m00, fc, al.m02), fmaf(al.m10, fc, al.m12));
         float h = 0.f;
 #pragma unroll
@@ -1316,7 +1317,8 @@ __global__ void __launch_bounds__(ADJ_PIXELS* ADJ_SPLIT) bp_adjoint_kernel(BpArg
           const float2 d = __fadd2_rn(__ffma2_rn(make_float2(al.m01, al.m11), fr[dr], pc), make_float2(-fj, -fi));
           h = fmaf(fmaxf(1.f - fabsf(d.x), 0.f), fmaxf(1.f - fabsf(d.y), 0.f), h);
         }
-        lsum += (double)h * (double)__ldg(y + c);
+        // a bin that does not reach the pixel adds nothing, whatever it holds
+        lsum = fma((double)h, h > 0.f ? (double)yc : 0.0, lsum);
       }
       double contrib = lsum * al.w;
       if (HAS_MAPS) {

@@ -34,3 +34,26 @@ def test_adjoint_matches_port(n, n_ang, n_det):
     if n_det == 1:
         got = c.bp(torch.from_numpy(y).to(dev), "adjoint").double().cpu().numpy()
         assert rel_l2(got[1], port.fp_xrf_adjoint(y[1, 0].astype(np.float64), None, deg32, n)) < TOL
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("n,angle", [(9, 0.0), (33, 0.3), (33, np.pi / 4), (64, 2.0), (71, np.pi / 2)])
+def test_adjoint_keeps_a_bad_bin_to_its_pixels(n, angle, bad):
+    """A bin that is not finite reaches the pixels that a bin of 1 reaches, and no others (candidates past
+    the reach of the hats, or on lattice rows outside the image, add nothing)."""
+    from oracle import port
+    from pycorrectedemissionct_b200 import core
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    dev = torch.device("cuda", 0)
+    c = core.XrfCore(n, [angle], device=dev)
+    _, deg32 = port.backend_angles(np.array([angle]))
+    for k in (0, 1, n // 2, n - 1):
+        y = torch.zeros((1, 1, 1, n), device=dev)
+        y[..., k] = 1.0
+        one = c.bp(y, "adjoint")
+        ref = port.fp_xrf_adjoint(y[0, 0].double().cpu().numpy(), None, deg32, n)
+        assert np.abs(one[0].double().cpu().numpy() - ref).max() < 1e-4
+        y[..., k] = bad
+        assert torch.equal(torch.isfinite(c.bp(y, "adjoint")), one == 0.0)

@@ -1237,8 +1237,9 @@ __global__ void __launch_bounds__(BP_THREADS, 4) bp_ragged_kernel(const BpArgs* 
 //
 // Bound: issue (~110 instructions per pixel and line for the nine candidates).  A CTA holds 64 pixels
 // and four threads of each take every fourth line, since one thread per pixel leaves most of the
-// chip's warps empty at 256^2.  256^2 x 360: 1134 us with 36 candidates in FP64 per thread and
-// line, 211 us so.  The line sums and the sum over lines stay FP64.
+// chip's warps empty at 256^2.  Positions and hats are FP32 like the forward's; the products of two
+// hats and all sums are FP64 (253 us; with FP32 products and column sums 230 us, with their errors
+// carried along in FP32 279 us).  256^2 x 360 with 36 candidates per thread and line: 1170 us.
 // ------------------------------------------------------------------------------------------
 constexpr int ADJ_PIXELS = 64;
 constexpr int ADJ_SPLIT = 4;
@@ -1310,15 +1311,15 @@ __global__ void __launch_bounds__(ADJ_PIXELS* ADJ_SPLIT) bp_adjoint_kernel(BpArg
         if ((unsigned)c >= (unsigned)n) continue;
         const float yc = __ldg(y + c);
         const float2 pc = make_float2(fmaf(al.m00, fc, al.m02), fmaf(al.m10, fc, al.m12));
-        float h = 0.f;
+        double h = 0.0;
 #pragma unroll
         for (int dr = 0; dr < 3; ++dr) {
           // same float arithmetic as the forward kernel's sample position (sample_x)
           const float2 d = __fadd2_rn(__ffma2_rn(make_float2(al.m01, al.m11), fr[dr], pc), make_float2(-fj, -fi));
-          h = fmaf(fmaxf(1.f - fabsf(d.x), 0.f), fmaxf(1.f - fabsf(d.y), 0.f), h);
+          h = fma((double)fmaxf(1.f - fabsf(d.x), 0.f), (double)fmaxf(1.f - fabsf(d.y), 0.f), h);
         }
         // a bin that does not reach the pixel adds nothing, whatever it holds
-        lsum = fma((double)h, h > 0.f ? (double)yc : 0.0, lsum);
+        lsum = fma(h, h > 0.0 ? (double)yc : 0.0, lsum);
       }
       double contrib = lsum * al.w;
       if (HAS_MAPS) {

@@ -57,3 +57,28 @@ def test_adjoint_keeps_a_bad_bin_to_its_pixels(n, angle, bad):
         assert np.abs(one[0].double().cpu().numpy() - ref).max() < 1e-4
         y[..., k] = bad
         assert torch.equal(torch.isfinite(c.bp(y, "adjoint")), one == 0.0)
+
+
+@pytest.mark.parametrize("n,angle", [(9, 0.2), (33, 0.9), (64, 2.0), (71, 3.5)])
+def test_adjoint_forms_hat_products_in_double(n, angle):
+    """One bin of 1: a pixel is the sum of the products of its samples' FP32 hats, formed in FP64 and rounded to
+    FP32 once; the FP32 positions are mirrored here, so the results are equal."""
+    from oracle import port
+    from test_host import _fma32
+    from pycorrectedemissionct_b200 import core, geometry
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    dev = torch.device("cuda", 0)
+    f = np.float32
+    _, deg32 = port.backend_angles(np.array([angle]))
+    m00, m01, m02, m10, m11, m12 = geometry.fp_matrices(deg32, n)[0]
+    c = core.XrfCore(n, [angle], device=dev)
+    r, axis = np.arange(n, dtype=f)[:, None], np.arange(n, dtype=f)[None, :]
+    for k in (0, n // 2, n - 1):
+        y = torch.zeros((1, 1, 1, n), device=dev)
+        y[..., k] = 1.0
+        hx = np.maximum(f(1) - np.abs(_fma32(m01, r, _fma32(m00, f(k), m02)) - axis), f(0)).astype(np.float64)
+        hy = np.maximum(f(1) - np.abs(_fma32(m11, r, _fma32(m10, f(k), m12)) - axis), f(0)).astype(np.float64)
+        want = (hy.T @ hx).astype(f)
+        assert np.array_equal(c.bp(y, "adjoint")[0].cpu().numpy(), want)

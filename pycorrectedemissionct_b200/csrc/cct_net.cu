@@ -156,10 +156,13 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
                : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
+// (.aligned: the whole warp takes part, joined here after its lanes' own branches)
 __device__ __forceinline__ void tmem_dealloc(uint32_t base, uint32_t cols) {
+  __syncwarp();
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols) : "memory");
 }
 __device__ __forceinline__ void tmem_load16(uint32_t addr, uint32_t (&r)[16]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
       "[%16];"
@@ -375,9 +378,9 @@ __global__ void __launch_bounds__(CONV_THREADS)
         __nv_bfloat16* out = a.y + (((int64_t)i.b * a.h + y) * a.w + x) * a.cout + n0;
 #pragma unroll 1
         for (int c0 = c_begin; c0 < c_end; c0 += 16) {
+          if (n0 + c0 >= a.cout) break;  // the whole warp
           uint32_t r[16];
           tmem_load16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((buf * MT + m) * bn + c0), r);
-          if (!in || n0 + c0 >= a.cout) continue;
           uint32_t o[8];
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
@@ -390,11 +393,11 @@ __global__ void __launch_bounds__(CONV_THREADS)
             const __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
             o[k] = *reinterpret_cast<const uint32_t*>(&h);
           }
-          if (a.wide) {
+          if (in && a.wide) {
             asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(out + c0), "r"(o[0]), "r"(o[1]),
                          "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7])
                          : "memory");
-          } else {
+          } else if (in) {
             reinterpret_cast<uint4*>(out + c0)[0] = make_uint4(o[0], o[1], o[2], o[3]);
             reinterpret_cast<uint4*>(out + c0)[1] = make_uint4(o[4], o[5], o[6], o[7]);
           }

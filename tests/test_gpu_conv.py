@@ -106,3 +106,53 @@ def test_convolutions_of_one_tap_per_stage(b, h, w, cin, cout):
     """Several channel blocks with weights that stay in shared memory (9 cin cout values in 74 KB at most) and
     one block with weights that do not: both walk the taps one by one."""
     test_convolutions_at_tile_edges(b, h, w, cin, cout)
+
+
+@pytest.mark.parametrize("cin,cout,offset", [(16, 16, 0), (32, 32, 0), (64, 64, 0), (64, 48, 8), (128, 16, 0), (64, 128, 0),
+                                             (128, 144, 8), (256, 32, 0)])
+def test_persistent_tiles_reuse_their_buffers(cin, cout, offset):
+    """At least five tiles per CTA with ragged edges, so that every ring of stages wraps and both accumulators
+    are filled again: whole tiles of 16, 32 and 64 channels, one tap per stage with weights that stay
+    (128 -> 16) and that do not, the weight gradient with one, two and three sets of taps, and results
+    that begin at 16, not 32 bytes.  Lanes past the image store nothing."""
+    from pycorrectedemissionct_b200 import _lib
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    dev = torch.device("cuda", 0)
+    lib = _lib.load()
+    b, h, w = 2, 227, 397
+    g = torch.Generator(device=dev)
+    g.manual_seed(cin + cout)
+    x = torch.randn((b, h, w, cin), generator=g, device=dev).bfloat16()
+    wt = (torch.randn((cout, 9, cin), generator=g, device=dev) / (3 * cin**0.5)).bfloat16()
+    dy = torch.randn((b, h, w, cout), generator=g, device=dev).bfloat16()
+    bias = torch.randn(cout, generator=g, device=dev)
+    buf = torch.full((b * h * w * cout + 2 * offset + 32,), float("nan"), device=dev, dtype=torch.bfloat16)
+    y = buf[offset:offset + b * h * w * cout].view(b, h, w, cout)
+    assert y.data_ptr() % 32 == (16 if offset else 0)
+    dw = torch.zeros((cout, 9, cin), device=dev)
+    d = _lib.ConvDesc(b, h, w, cin, cout)
+    _lib.check(lib.cct_conv3x3_fwd(ctypes.byref(d), x.data_ptr(), wt.data_ptr(), bias.data_ptr(), 0, y.data_ptr(), None))
+    _lib.check(lib.cct_conv3x3_wgrad(ctypes.byref(d), x.data_ptr(), dy.data_ptr(), dw.data_ptr(), None))
+    torch.cuda.synchronize()
+    ref = F.conv2d(x.double().permute(0, 3, 1, 2), wt.double().reshape(cout, 3, 3, cin).permute(0, 3, 1, 2),
+                   bias.double(), padding=1).permute(0, 2, 3, 1)
+    assert float((y.double() - ref).norm() / ref.norm()) < TOL_BF16
+    # every tile, not the whole: BF16 rounding and nothing else at each value
+    assert bool(((y.double() - ref).abs() <= 2.0**-8 * ref.abs() + 1e-3).all())
+    assert bool(torch.isnan(buf[:offset]).all()) and bool(torch.isnan(buf[offset + y.numel():]).all())
+    xp = F.pad(x.double().permute(0, 3, 1, 2), (1, 1, 1, 1))
+    rows = dy.double().permute(3, 0, 1, 2).reshape(cout, -1)
+    ref = torch.stack([rows @ xp[:, :, ky:ky + h, kx:kx + w].permute(0, 2, 3, 1).reshape(-1, cin)
+                       for ky in range(3) for kx in range(3)], 1)
+    assert float((dw.double() - ref).norm() / ref.norm()) < TOL_F32
+    v = ctypes.c_int32(0)
+    _lib.check(lib.cct_net_timeout(1, ctypes.byref(v)))
+    assert v.value == 0
+
+
+def test_bias_gradient_of_several_channel_blocks():
+    """More than 256 channels one by one (an address that does not allow 16-byte loads): several blocks of
+    channels along the grid."""
+    test_elementwise_wide_and_narrow(520, 1)

@@ -136,6 +136,16 @@ __device__ __forceinline__ bool net_mbar_wait(uint64_t* bar, uint32_t phase, vol
   return false;
 }
 
+// After a CTA gave up: waits (bounded each) until the last use of every barrier of a ring is complete, `uses`
+// being the uses of the ring so far, so that no copy or MMA in flight outlives its shared memory or TMEM.
+__device__ __noinline__ void net_drain(uint64_t* bars, int ring, int uses) {
+  int none = 0;
+  for (int k = 0; k < ring && k < uses; ++k) {
+    const int idx = uses - 1 - k;
+    net_mbar_wait(&bars[idx % ring], (uint32_t)((idx / ring) & 1), &none);
+  }
+}
+
 __device__ __forceinline__ void tma_4d(void* dst, const CUtensorMap* map, int c, int x, int y, int b, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
@@ -251,6 +261,7 @@ __global__ void __launch_bounds__(CONV_THREADS)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_sh;
+  int sent = 0, issued = 0;  // boxes' stages of the loading thread, stages consumed by the MMA thread
 
   if (warp == 0 && lane == 0) {
     // ---- loads
@@ -260,7 +271,7 @@ __global__ void __launch_bounds__(CONV_THREADS)
         for (int t = 0; t < 9; ++t)
           tma_3d(net_smem + w_base + (uint32_t)(c * 9 + t) * w_bytes, &tm_w, c * ck, t, 0, &w_full);
     }
-    int s = 0, sent = 0;
+    int s = 0;
     uint32_t phase = 0;
     bool ok = true;
     for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
@@ -288,18 +299,10 @@ __global__ void __launch_bounds__(CONV_THREADS)
         }
       }
     }
-    if (!ok) {
-      // the copies in flight land before shared memory goes (bounded; abort no longer cuts it short)
-      int none = 0;
-      for (int k = 0; k < a.stages && k < sent; ++k) {
-        const int idx = sent - 1 - k;
-        net_mbar_wait(&full[idx % a.stages], (uint32_t)((idx / a.stages) & 1), &none);
-      }
-    }
   } else if (warp == 1 && lane == 0) {
     // ---- MMAs
     const uint32_t idesc = umma_idesc(bn, false), hi = umma_desc_hi(CK), base = net_smem_u32(net_smem);
-    int s = 0, done = 0, issued = 0;
+    int s = 0, done = 0;
     uint32_t phase = 0;
     bool ok = true;
     if (a.resident && blockIdx.x < items) ok = net_mbar_wait(&w_full, 0, abort);
@@ -354,10 +357,6 @@ __global__ void __launch_bounds__(CONV_THREADS)
       }
       if (ok) umma_commit(&acc_full[buf]);
     }
-    if (*abort && issued > 0) {  // the MMAs in flight end before their operands and TMEM go
-      int none = 0;
-      net_mbar_wait(&empty[(issued - 1) % a.stages], (uint32_t)(((issued - 1) / a.stages) & 1), &none);
-    }
   } else if (warp >= 2) {
     // ---- results: TMEM lane = pixel, warp % 4 selects its 32 lanes
     const int quarter = warp & 3, half = (warp - 2) >> 2;
@@ -410,6 +409,12 @@ __global__ void __launch_bounds__(CONV_THREADS)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (abort_sh != 0) {  // whichever role gave up (all have ended, so abort no longer changes)
+    if (tid == 0 && a.resident && blockIdx.x < items) net_drain(&w_full, 1, 1);
+    if (tid == 0) net_drain(full, a.stages, sent);
+    if (tid == 32) net_drain(empty, a.stages, issued);
+    __syncthreads();
+  }
   if (warp == 1) tmem_dealloc(tmem, cols);
 }
 
@@ -470,17 +475,14 @@ __global__ void __launch_bounds__(CONV_THREADS)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_sh;
+  int sent = 0, issued = 0;  // as in the forward
 
   if (warp == 0 && lane == 0) {
-    int s = 0, sent = 0;
+    int s = 0;
     uint32_t phase = 0;
-    bool ok = true;
     for (int tile = t0; tile < t1; ++tile) {
       const int tx = tile % a.tiles_x, ty = (tile / a.tiles_x) % a.tiles_y, b = tile / (a.tiles_x * a.tiles_y);
-      if (sent >= a.stages && !net_mbar_wait(&empty[s], phase ^ 1u, abort)) {
-        ok = false;
-        break;
-      }
+      if (sent >= a.stages && !net_mbar_wait(&empty[s], phase ^ 1u, abort)) break;
       unsigned char* st = net_smem + (uint32_t)s * stage_bytes;
       net_mbar_expect(&full[s], a.bx * x_box + a.by * dy_box);
       for (int k = 0; k < a.bx; ++k)
@@ -493,13 +495,6 @@ __global__ void __launch_bounds__(CONV_THREADS)
         phase ^= 1u;
       }
     }
-    if (!ok) {
-      int none = 0;
-      for (int k = 0; k < a.stages && k < sent; ++k) {
-        const int idx = sent - 1 - k;
-        net_mbar_wait(&full[idx % a.stages], (uint32_t)((idx / a.stages) & 1), &none);
-      }
-    }
   } else if (warp == 1 && lane == 0) {
     const uint32_t idesc = umma_idesc(a.n, true);
     // along M the next ckx rows are the next vertical tap (one atom on), or the next box
@@ -507,16 +502,13 @@ __global__ void __launch_bounds__(CONV_THREADS)
     const uint32_t lbo_x = a.bx > 1 ? x_pitch : atom_x, lbo_y = a.by > 1 ? dy_box : atom_y;
     const uint32_t set_step = ((a.ckx == 64 && a.bx == 1 ? 2u : 1u) * atom_x) >> 4;
     const uint32_t hi_x = umma_desc_hi(a.ckx), hi_y = umma_desc_hi(a.cky);
-    int s = 0, issued = 0;
+    int s = 0;
     uint32_t phase = 0;
-    bool ok = true;
     for (int tile = t0; tile < t1; ++tile) {
       const int group = (tile - t0) / WGRAD_GROUP, in_group = (tile - t0) % WGRAD_GROUP, buf = group & 1;
       if ((in_group == 0 && group >= 2 && !net_mbar_wait(&acc_empty[buf], (uint32_t)(((group >> 1) & 1) ^ 1), abort)) ||
-          !net_mbar_wait(&full[s], phase, abort)) {
-        ok = false;
+          !net_mbar_wait(&full[s], phase, abort))
         break;
-      }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t d = tmem + (uint32_t)(buf * a.sets * a.n);
       const uint32_t xs = net_smem_u32(net_smem) + (uint32_t)s * stage_bytes;
@@ -538,10 +530,6 @@ __global__ void __launch_bounds__(CONV_THREADS)
         s = 0;
         phase ^= 1u;
       }
-    }
-    if (!ok && issued > 0) {
-      int none = 0;
-      net_mbar_wait(&empty[(issued - 1) % a.stages], (uint32_t)(((issued - 1) / a.stages) & 1), &none);
     }
   } else if (warp >= 2) {
     // a pair of warps per quarter of the lanes, each with every other block of 16 columns
@@ -589,6 +577,11 @@ __global__ void __launch_bounds__(CONV_THREADS)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (abort_sh != 0) {
+    if (tid == 0) net_drain(full, a.stages, sent);
+    if (tid == 32) net_drain(empty, a.stages, issued);
+    __syncthreads();
+  }
   if (warp == 1) tmem_dealloc(tmem, cols);
 }
 

@@ -736,3 +736,17 @@ def test_fp_fields_fill_keeps_every_tap_quad(n, n_angles):
                 gx, gy = (np.floor((x + dx) / 4) * 4).astype(f), (y + dy).astype(f)
                 assert abs(_fma32(i00, gx, _fma32(i01, gy, qc0))).max() <= hc
                 assert abs(_fma32(i10, gx, _fma32(i11, gy, qr0))).max() <= hr
+
+
+@pytest.mark.parametrize("ring", [1, 2, 3, 8])
+def test_convolution_drain_waits_for_every_last_use(ring):
+    """A convolution CTA that gives up waits for the last use of each barrier of its rings before it leaves
+    (net_drain in csrc/cct_net.cu): mirror the (barrier, parity) list against mbarrier phases.  A parity wait
+    returns once the phase in progress has the other parity; it has to hold while a barrier's last use is
+    outstanding and to return when it is complete, for every barrier that was used."""
+    for uses in range(4 * ring + 2):
+        waits = [((uses - 1 - k) % ring, ((uses - 1 - k) // ring) & 1) for k in range(min(ring, uses))]
+        used = {i % ring: i // ring + 1 for i in range(uses)}  # phases begun per barrier
+        assert sorted(b for b, _ in waits) == sorted(used)
+        for b, parity in waits:
+            assert (used[b] - 1) % 2 == parity and used[b] % 2 != parity

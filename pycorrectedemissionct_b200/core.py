@@ -389,11 +389,14 @@ def compute_maps(
     if use_quads:
         desc.quads, desc.n_quads, desc.emitted_scale = quads_d.data_ptr(), quads_d.shape[0], float(emitted_scale)
         entries = quads_d.shape[0]  # a quad takes one entry's workspace (two incident fields)
-    need = ctypes.c_size_t(0)
-    _lib.call("cct_maps_workspace_size", ctypes.byref(desc), 1, ctypes.byref(need))
+    size = ctypes.c_size_t(0)
+    _lib.call("cct_maps_workspace_size", ctypes.byref(desc), 1, ctypes.byref(size))
+    need = int(size.value)
+    own_out = mu_out is not None and not use_quads and (mu_in is None or mu_out.data_ptr() != mu_in.data_ptr())
+    copies = (int(mu_in is not None) + int(own_out)) * _maps_copy_bytes(n, s)
     if workspace is None:
-        # at least 8 angles (of the whole batch) per pass, at most all of them
-        nbytes = min(max(int(workspace_bytes), 8 * int(need.value)), int(need.value) * entries)
+        # beside the copies of mu, at least 8 angles (of the whole batch) per pass, at most all of them
+        nbytes = min(max(int(workspace_bytes), 8 * need + copies), need * entries + copies)
         workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
     planes = n_det + 1 if cdt == _lib.CCT_DTYPE_FIELDS_F32 else n_det
     if out is None:
@@ -401,7 +404,9 @@ def compute_maps(
     else:
         _check_tensor(out, (s, n_ang, planes, n, n), tdt, device, "out")
         maps = out
-    compute_maps.last_passes = -(-entries // max(1, (workspace.numel() * workspace.element_size()) // int(need.value)))
+    jobs = 2 if use_quads else desc.has_in + desc.has_out * n_det * n_sub
+    compute_maps.last_passes = -(-entries // _maps_entries_per_pass(
+        workspace.numel() * workspace.element_size(), need, entries, copies, jobs))
     _lib.call(
         "cct_compute_maps", ctypes.byref(desc), _ptr(mu_in), _ptr(mu_out), maps.data_ptr(), workspace.data_ptr(),
         workspace.numel() * workspace.element_size(), stream_handle(device),
@@ -415,6 +420,21 @@ def compute_maps(
     # torch's caching allocator reuses a workspace allocated here only for work queued later on
     # the same stream, so dropping it here is safe
     return maps
+
+
+def _maps_copy_bytes(n: int, n_slices: int) -> int:
+    """Workspace bytes of the copies that ``cct_compute_maps`` makes of one attenuation volume: transposed,
+    and with rows padded to 16 bytes where n % 4 != 0."""
+    one = -(-n * ((n + 3) // 4 * 4) * 4 * n_slices // 256) * 256
+    return one if n % 4 == 0 else 2 * one
+
+
+def _maps_entries_per_pass(nbytes: int, need: int, entries: int, copies: int, jobs: int) -> int:
+    """Entries that ``cct_compute_maps`` takes per pass of a workspace of ``nbytes``: beside the copies of
+    mu where at least half as many fit there, at most what its grids hold."""
+    plain = min(nbytes // need, entries)
+    beside = min(max(nbytes - copies, 0) // need, entries)
+    return max(1, min(beside if beside >= 1 and 2 * beside >= plain else plain, 65535 // jobs))
 
 
 def maps_entry_bytes(n: int, n_slices: int, n_det: int = 1, n_sub: int = 1, has_in: bool = True,

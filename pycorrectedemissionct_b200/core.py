@@ -41,9 +41,15 @@ def require_cuda(device=None) -> torch.device:
     return device
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # not public: may be missing
+
+
 def stream_handle(device: torch.device) -> int:
-    """The current stream's handle (the raw getter: building a ``torch.cuda.Stream`` takes ~3 us per call)."""
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
+    """The current stream's handle (by torch's raw getter where there is one: building a
+    ``torch.cuda.Stream`` takes ~3 us per call)."""
+    if _raw_stream is None or not isinstance(device, torch.device):
+        return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(torch.cuda.current_device() if device.index is None else device.index)
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:

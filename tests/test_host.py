@@ -750,3 +750,22 @@ def test_convolution_drain_waits_for_every_last_use(ring):
         assert sorted(b for b, _ in waits) == sorted(used)
         for b, parity in waits:
             assert (used[b] - 1) % 2 == parity and used[b] % 2 != parity
+
+
+def test_stream_handle_without_the_raw_getter(monkeypatch):
+    """stream_handle takes torch's private getter where it exists, and the public stream otherwise, also for the
+    devices that only the latter accepts (an index, a name)."""
+    import types
+
+    import torch
+
+    from pycorrectedemissionct_b200 import core
+
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda d: types.SimpleNamespace(cuda_stream=("public", d)))
+    monkeypatch.setattr(core, "_raw_stream", lambda index: ("raw", index))
+    assert core.stream_handle(torch.device("cuda", 1)) == ("raw", 1)
+    assert core.stream_handle(torch.device("cuda")) == ("raw", 3)
+    assert core.stream_handle(2) == ("public", 2) and core.stream_handle("cuda:2") == ("public", "cuda:2")
+    monkeypatch.setattr(core, "_raw_stream", None)
+    assert core.stream_handle(torch.device("cuda", 1)) == ("public", torch.device("cuda", 1))

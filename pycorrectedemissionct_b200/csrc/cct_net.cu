@@ -947,6 +947,7 @@ static bool ew_wide(const void* a, const void* b, const void* d, int64_t c) {
 // small (h x w) and large (2h x 2w) images of c channels
 static void launch_resize2(const void* src, void* dst, int64_t rows, int w, int c, int half, bool to_small,
                            cudaStream_t st) {
+  if (rows <= 0 || w <= 0) return;  // empty images: nothing to do
   const bool wide = ew_wide(src, dst, nullptr, c);
   const int per_row = w * (wide ? c / 8 : c);
   const dim3 grid((unsigned)std::min(64, (per_row + 255) / 256), (unsigned)std::min<int64_t>(rows, 65535));

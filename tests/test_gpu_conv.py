@@ -156,3 +156,19 @@ def test_bias_gradient_of_several_channel_blocks():
     """More than 256 channels one by one (an address that does not allow 16-byte loads): several blocks of
     channels along the grid."""
     test_elementwise_wide_and_narrow(520, 1)
+
+
+@pytest.mark.parametrize("h,w", [(0, 4), (4, 0), (0, 0)])
+def test_pooling_of_empty_images(h, w):
+    """Images without rows or columns are accepted and nothing is written, both ways."""
+    from pycorrectedemissionct_b200 import _lib
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    lib = _lib.load()
+    x = torch.ones(64, device="cuda", dtype=torch.bfloat16)
+    y = torch.full((64,), 3.0, device="cuda", dtype=torch.bfloat16)
+    for backward in (0, 1):
+        _lib.check(lib.cct_net_avgpool2(x.data_ptr(), y.data_ptr(), 1, h, w, 16, backward, None))
+    torch.cuda.synchronize()
+    assert bool((y == 3.0).all())

@@ -1095,14 +1095,12 @@ __device__ __forceinline__ void bp_segment(const BpArgs& args, BpShared& sh, int
 #pragma unroll
         for (int k = 0; k < PPT; k += 2) {
           const float2 u = __ffma2_rn(nfi[k / 2], sn2, base2);
-          float2 r = bp_lerp2(pairs, row, u);
+          const float2 r = bp_lerp2(pairs, row, u);
           const bool e0 = fabsf(fabsf(u.x - mid) - half) < BP_EDGE_GUARD;
           const bool e1 = fabsf(fabsf(u.y - mid) - half) < BP_EDGE_GUARD;
-          if (e0) r.x = 0.f;
-          if (e1) r.y = 0.f;
           any = any || e0 || e1;
-          acc[k] = SYM ? acc[k] + r.x * m[k] : acc[k] + r.x;
-          acc[k + 1] = SYM ? acc[k + 1] + r.y * m[k + 1] : acc[k + 1] + r.y;
+          if (!e0) acc[k] = SYM ? acc[k] + r.x * m[k] : acc[k] + r.x;
+          if (!e1) acc[k + 1] = SYM ? acc[k + 1] + r.y * m[k + 1] : acc[k + 1] + r.y;
         }
         if (any) near_edge |= 1u << ll;
       }

@@ -95,3 +95,22 @@ def test_bp_interpolates_edge_pixels_in_double(n):
         assert np.all(np.abs(got + d)[near] <= 1e-11 + 2.0**-24 * d[near])
         checked += int(near.sum())
     assert checked > 0
+
+
+@pytest.mark.parametrize("n_ang", [1, 16])
+@pytest.mark.parametrize("n", [33, 64])
+def test_symmetric_bp_of_unbounded_maps_at_the_edges(n, n_ang):
+    """A map value of infinity makes its pixel infinite, on the detector's edge bins (angle 0: the first and last
+    columns) as inside."""
+    from pycorrectedemissionct_b200 import core
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    dev = torch.device("cuda", 0)
+    c = core.XrfCore(n, np.zeros(n_ang), device=dev)
+    y = torch.ones((1, 1, n_ang, n), device=dev)
+    maps = torch.ones((1, n_ang, 1, n, n), device=dev)
+    want = torch.full((1, n, n), float(n_ang), device=dev)
+    for i, j in ((0, 0), (1, n - 1), (n // 2, n // 3), (n - 1, n - 1)):
+        maps[0, n_ang // 2, 0, i, j] = want[0, i, j] = float("inf")
+    assert torch.equal(c.bp(y, "symmetric", maps), want)

@@ -879,6 +879,7 @@ __host__ __device__ inline int bp_log2_segments(int n_lines) {
 }
 
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();  // .aligned takes whole warps, also after stores that depend on the pixel
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 

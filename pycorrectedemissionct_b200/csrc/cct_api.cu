@@ -413,6 +413,7 @@ int cct_ragged_plan_create(int32_t method, int32_t bp_mode, int32_t n_groups, co
     return code;
   };
   fps[0] = bps[0] = rss[0] = 0;
+  int64_t tiles64 = 0;
   for (int g = 0; g < n_groups; ++g) {
     const cct_xrf_desc* d = descs + g;
     const cct_solver_state* st = states + g;
@@ -449,10 +450,13 @@ int cct_ragged_plan_create(int32_t method, int32_t bp_mode, int32_t n_groups, co
     const int64_t per_slice = bands * d->n_angles * d->n_det;
     res[g] = cct::ResidualGroup{st->partials, per_slice, st->residuals, st->active, st->iterations, st->tolerance,
                                 st->residual_history, st->history_len};
-    const int64_t tiles = cct::bp_tile_count(d->n);
     fps[g + 1] = fps[g] + per_slice * d->n_slices;
-    bps[g + 1] = bps[g] + tiles * d->n_slices;
     rss[g + 1] = rss[g] + d->n_slices;
+    tiles64 += cct::bp_tile_count(d->n, 64) * d->n_slices;
+  }
+  for (int g = 0; g < n_groups; ++g) {
+    bp[g].tile_rows = cct::bp_ragged_tile_rows(bp[g].n, tiles64);
+    bps[g + 1] = bps[g] + cct::bp_tile_count(bp[g].n, bp[g].tile_rows) * bp[g].n_slices;
   }
   p->fp_ctas = fps[n_groups];
   p->bp_ctas = bps[n_groups];

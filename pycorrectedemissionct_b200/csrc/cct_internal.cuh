@@ -65,6 +65,7 @@ struct BpArgs {
   float lower, upper;
   int has_lower, has_upper;
   const int* active;
+  int tile_rows;           // rows of a tile: set by launch_bp, for ragged groups with their tile offsets
 };
 
 // Fused forward-projection epilogue for one final value `ax` = (A x)[idx].
@@ -197,14 +198,15 @@ bool fp_vec4_ok(const FpArgs& a);  // may the fp staging use 16-byte loads for t
 void launch_psf(const FpArgs& a, const float* psf, int psf_len, cudaStream_t st);
 int read_device_error(int clear, int* value);
 void launch_bp(const BpArgs& a, cudaStream_t st);
-int64_t bp_tile_count(int n);  // pixel tiles of one slice
+int64_t bp_tile_count(int n, int tile_rows);        // pixel tiles of one slice
+int bp_ragged_tile_rows(int n, int64_t tiles64);    // tile_rows of a group of side n in a ragged launch of tiles64 tiles of 64 rows
 
 // Ragged launches: one grid over groups of slices (tables in device memory, CTA offsets
 // start[0..n_groups], start[n_groups] = total CTAs).  Every group shares the epilogue, the
 // presence and the storage type of the maps (and, for bp, the mode).
 void launch_fp_ragged(const FpArgs* groups, const int64_t* start, int n_groups, int64_t ctas, int epi, bool has_maps,
                       int maps_dtype, cudaStream_t st);
-// (bp: start holds tile offsets, launched as one CTA or one cluster per tile)
+// (bp: start holds offsets of tiles of the groups' tile_rows, launched as one CTA or one cluster per tile)
 void launch_bp_ragged(const BpArgs* groups, const int64_t* start, int n_groups, int64_t ctas, int epi, bool sym,
                       int maps_dtype, cudaStream_t st);
 

@@ -842,7 +842,7 @@ __global__ void __launch_bounds__(FP_THREADS, 4) fp_pair_kernel(FpArgs args) {
 // ------------------------------------------------------------------------------------------
 // Back projection (reference iradon discretisation, optional maps x weights)
 //
-// A CTA owns a 32-column tile of TI = 32 or 64 rows; a warp holds TI / 8 whole rows of it.
+// A CTA owns a 32-column tile of TI = 32 or 64 rows (bp_tile_rows); a warp holds TI / 8 whole rows of it.
 //
 // Bound: an 8-byte lookup is two shared-memory wavefronts whatever the lanes' pixels (0.40 ms of
 // them for 8 slices of 512^2 x 720), next the ~8 instructions per pixel and line.  What else
@@ -858,6 +858,8 @@ __global__ void __launch_bounds__(FP_THREADS, 4) fp_pair_kernel(FpArgs args) {
 // combine them through distributed shared memory; both give the same bits.
 // ------------------------------------------------------------------------------------------
 constexpr int BP_TJ = 32;                                // tile columns
+constexpr int BP_BLOCK_ROWS = 64;                        // rows of the blocks whose bins are staged
+constexpr int BP_MAX_RANKS = 8;                          // CTAs of a cluster, at most, and in a ragged launch
 constexpr int BP_THREADS = 256;
 constexpr int BP_LINES = 16;                             // lines staged per chunk
 constexpr int BP_KW = 80;                                // staged pairs per line (>= 74 needed)
@@ -865,12 +867,9 @@ constexpr float BP_EDGE_GUARD = 0.01f;
 
 enum : int { LINE_FAST = 0, LINE_CHECKED = 1, LINE_EMPTY = 2 };
 
-// Rows of a tile: small images take smaller tiles for more CTAs.  (The rounding of a pixel's bin
-// depends on its tile, so the choice depends on n alone.)
-__host__ __device__ inline int bp_tile_rows(int n) { return n > 192 ? 64 : 32; }
-__host__ __device__ inline int bp_tiles(int n) {
-  const int ti = bp_tile_rows(n);
-  return ((n + BP_TJ - 1) / BP_TJ) * ((n + ti - 1) / ti);
+// Tiles of a slice with tiles of `rows` rows.
+__host__ __device__ inline int bp_tiles(int n, int rows) {
+  return ((n + BP_TJ - 1) / BP_TJ) * ((n + rows - 1) / rows);
 }
 // log2 of the segments of the line sum (at least eight lines each); segment g of n_lines <= 65535
 // lines starts at (g * n_lines) >> log2.
@@ -951,7 +950,6 @@ template <bool SYM, int MAPS_DTYPE, int PPT>
 __device__ __forceinline__ void bp_segment(const BpArgs& args, BpShared& sh, int s, int ti0, int tj0, int i0, int j,
                                            int l0, int l1, float (&acc)[PPT]) {
   static_assert(PPT % 2 == 0 && BP_LINES <= 32, "pixels go in pairs, lines in one mask");
-  constexpr int TI = 8 * PPT;
   const int n = args.n;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int K = n / 2;  // detector offset (img_shape // 2) and output radius (output_size // 2)
@@ -980,9 +978,11 @@ __device__ __forceinline__ void bp_segment(const BpArgs& args, BpShared& sh, int
     const int d = l / args.n_angles;
     const int a = l - d * args.n_angles;
     // full tile (also pixels beyond n, which are computed and discarded) so every thread's lookup
-    // stays inside the staged range: t = (j - K) cos - (i - K) sin at the four corners
+    // stays inside the staged range: t = (j - K) cos - (i - K) sin at the four corners (of the block of 64
+    // rows, whatever the tile's: a pixel's bin is rounded from there, and so the same in both)
+    const int b0 = ti0 & ~(BP_BLOCK_ROWS - 1);
     const float cj0 = (float)(tj0 - K), cj1 = (float)(tj0 + BP_TJ - 1 - K);
-    const float ci0 = (float)(ti0 - K), ci1 = (float)(ti0 + TI - 1 - K);
+    const float ci0 = (float)(b0 - K), ci1 = (float)(b0 + BP_BLOCK_ROWS - 1 - K);
     BpLine li;
     li.cs = args.bp_trig[2 * a];
     li.sn = args.bp_trig[2 * a + 1];
@@ -1192,7 +1192,7 @@ __device__ __forceinline__ void bp_tile(const BpArgs& args, BpShared& sh, int ti
 template <int EPI, bool SYM, int MAPS_DTYPE, bool CLUSTER>
 __device__ __forceinline__ void bp_cta(const BpArgs& args, int tile, int s, int rank, int ranks) {
   __shared__ __align__(16) BpShared sh;
-  if (bp_tile_rows(args.n) == 64) {
+  if (args.tile_rows == BP_BLOCK_ROWS) {
     bp_tile<EPI, SYM, MAPS_DTYPE, 8, CLUSTER>(args, sh, tile, s, rank, ranks);
   } else {
     bp_tile<EPI, SYM, MAPS_DTYPE, 4, CLUSTER>(args, sh, tile, s, rank, ranks);
@@ -1213,8 +1213,6 @@ __global__ void __launch_bounds__(BP_THREADS, 4) bp_cluster_kernel(BpArgs args, 
 
 // Back projection over groups of slices in one launch: group g's tiles are (tile, slice), tile
 // fastest, each one CTA or one cluster of BP_MAX_RANKS CTAs (CLUSTER).
-constexpr int BP_MAX_RANKS = 8;
-
 template <int EPI, bool SYM, int MAPS_DTYPE, bool CLUSTER>
 __global__ void __launch_bounds__(BP_THREADS, 4) bp_ragged_kernel(const BpArgs* __restrict__ groups,
                                                                   const int64_t* __restrict__ start, int n_groups) {
@@ -1222,7 +1220,7 @@ __global__ void __launch_bounds__(BP_THREADS, 4) bp_ragged_kernel(const BpArgs* 
   const int64_t cta = blockIdx.x / RANKS;
   const int g = ragged_group(start, n_groups, cta);
   const BpArgs& a = groups[g];
-  const int tiles = bp_tiles(a.n);
+  const int tiles = bp_tiles(a.n, a.tile_rows);
   const int64_t local = cta - start[g];
   bp_cta<EPI, SYM, MAPS_DTYPE, CLUSTER>(a, (int)(local % tiles), (int)(local / tiles), blockIdx.x % RANKS, RANKS);
 }
@@ -1518,13 +1516,24 @@ static void launch_cluster(Kernel kernel, const dim3& grid, int ranks, cudaStrea
 }
 
 // Tiles of a batch below which the CTAs of a cluster share each tile's lines: the crossing lies between
-// two and three tiles per SM (512^2 x 720: 327 us in clusters, 333 without at 3 slices = 384 tiles, 422
-// and 414 at 4; 256^2 x 360: 144 and 157 at 8 slices = 256 tiles, 203 and 182 at 12).
+// two and four tiles per SM (512^2 x 720: 327 us in clusters, 333 without at 3 slices = 384 tiles, 422
+// and 414 at 4; 256^2 x 360: 144 and 157 at 8 slices = 256 tiles, 203 and 182 at 12; 128^2 x 180: 64 and 72
+// at 32 slices = 256 tiles, 118 and 119 at 64).
 constexpr int64_t BP_FEW_TILES = 352;
 
+// Rows of a batch's tiles (one CTA or, with `segs` > 1, a cluster of as many for each).  A tile of 64 rows
+// stages a line for twice the pixels; tiles of 32 rows pay while their CTAs leave most of the chip idle
+// and a tile's own time counts: up to two per SM in clusters (128^2 x 180: 10.6 us with 32 rows, 11.8 with 64
+// at 1 slice = 128 CTAs, 15.9 and 14.1 at 4 slices = 512), up to four per SM with one segment (192^2 x 4:
+// 6.7 and 7.7 us at 16 slices = 576 CTAs, 10.6 and 9.8 at 32).  Large batches gain most from 64 rows
+// (128^2 x 180, 1024 slices: 2020 and 1338 us).
+static int bp_tile_rows(int64_t tiles32, int segs) { return tiles32 * segs <= (segs > 1 ? 296 : 592) ? 32 : BP_BLOCK_ROWS; }
+
 template <int EPI, bool SYM, int MAPS_DTYPE>
-static void launch_bp_inst(const BpArgs& a, cudaStream_t st) {
-  const int tiles = bp_tiles(a.n), segs = 1 << bp_log2_segments(a.n_det * a.n_angles);
+static void launch_bp_inst(BpArgs a, cudaStream_t st) {
+  const int segs = 1 << bp_log2_segments(a.n_det * a.n_angles);
+  a.tile_rows = bp_tile_rows((int64_t)bp_tiles(a.n, 32) * a.n_slices, segs);
+  const int tiles = bp_tiles(a.n, a.tile_rows);
   if (segs > 1 && (int64_t)tiles * a.n_slices < BP_FEW_TILES) {
     launch_cluster(bp_cluster_kernel<EPI, SYM, MAPS_DTYPE>, dim3(tiles * segs, a.n_slices), segs, st, a, segs);
   } else {
@@ -1593,7 +1602,12 @@ static void launch_bp_ragged_epi(const BpArgs* g, const int64_t* start, int ng, 
   }
 }
 
-int64_t bp_tile_count(int n) { return bp_tiles(n); }
+int64_t bp_tile_count(int n, int rows) { return bp_tiles(n, rows); }
+
+// A ragged launch ends with its longest tiles: up to four waves of tiles of 64 rows (4 x 592) the small sides,
+// which often have the most lines, keep 32 (eight groups of 128^2 x 360 to 512^2 x 90, 2 slices each: SIRT
+// step 1038 us, 1124 with 64 rows); with more the rows' own cost counts, as above.
+int bp_ragged_tile_rows(int n, int64_t tiles64) { return n <= 192 && tiles64 < 2368 ? 32 : BP_BLOCK_ROWS; }
 
 void launch_bp_ragged(const BpArgs* groups, const int64_t* start, int n_groups, int64_t ctas, int epi, bool sym,
                       int maps_dtype, cudaStream_t st) {

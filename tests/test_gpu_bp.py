@@ -114,3 +114,27 @@ def test_symmetric_bp_of_unbounded_maps_at_the_edges(n, n_ang):
     for i, j in ((0, 0), (1, n - 1), (n // 2, n // 3), (n - 1, n - 1)):
         maps[0, n_ang // 2, 0, i, j] = want[0, i, j] = float("inf")
     assert torch.equal(c.bp(y, "symmetric", maps), want)
+
+
+@pytest.mark.parametrize("n_ang", [4, 20, 70])
+@pytest.mark.parametrize("n", [31, 33, 64, 96, 130, 192, 200])
+def test_bp_tile_rows_and_clusters_give_the_same_bits(n, n_ang):
+    """Tiles of 32 and of 64 rows, in clusters and not: batches on all sides of both rules hold the slice of a
+    batch of one, in the reference and the symmetric mode."""
+    from pycorrectedemissionct_b200 import core
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    dev = torch.device("cuda", 0)
+    tiles32, tiles64 = ((n + 31) // 32) ** 2, (n + 31) // 32 * ((n + 63) // 64)
+    segs = 8 if n_ang >= 64 else 2 if n_ang >= 16 else 1
+    few = (296 if segs > 1 else 592) // segs // tiles32  # the last batch of 32-row tiles
+    batches = sorted({1, few, few + 1, 351 // tiles64, 352 // tiles64 + 1} - {0})
+    g = torch.Generator(device=dev).manual_seed(n * n_ang)
+    y = torch.rand((batches[-1], 1, n_ang, n), device=dev, generator=g)
+    maps = torch.rand((1, n_ang, 1, n, n), device=dev, generator=g).expand(batches[-1], -1, -1, -1, -1).contiguous()
+    c = core.XrfCore(n, np.linspace(0, 2 * np.pi, n_ang, endpoint=False), device=dev)
+    ref, sym = c.bp(y[:1]), c.bp(y[:1], "symmetric", maps[:1])
+    for s in batches[1:]:
+        assert torch.equal(c.bp(y[:s])[:1], ref) and torch.equal(c.bp(y[:s].flip(0).contiguous())[-1:], ref)
+        assert torch.equal(c.bp(y[:s], "symmetric", maps[:s])[:1], sym)

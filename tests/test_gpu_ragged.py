@@ -98,3 +98,26 @@ def test_ragged_rejects_mixed_groups(cuda):
         engine.RaggedSolvers([engine.BatchedSolver(c1, m1, b1, "mlem"), engine.BatchedSolver(c2, m2, b2, "mlem")])
     with pytest.raises(ValueError):
         engine.RaggedSolvers([engine.BatchedSolver(c1, m1, b1, "mlem"), engine.BatchedSolver(c1, m1, b1, "sirt")])
+
+
+@pytest.mark.parametrize("method", ["mlem", "sirt"])
+@pytest.mark.parametrize("slices", [(1, 1), (2, 1100), (400, 40)])
+def test_ragged_tile_rows(slices, method, cuda):
+    """Groups of small sides in launches of few tiles (tiles of 32 rows, clusters), of many (no clusters) and of
+    more than four waves (tiles of 64 rows): equal to stepping every group on its own."""
+    from pycorrectedemissionct_b200 import core, engine
+
+    g = torch.Generator(device=cuda).manual_seed(5)
+    pairs = []
+    for (n, n_ang), s in zip(((96, 20), (40, 6)), slices):
+        c = core.XrfCore(n, np.linspace(0, 2 * np.pi, n_ang, endpoint=False), device=cuda)
+        maps = torch.rand((1, n_ang, 1, n, n), device=cuda, generator=g).expand(s, -1, -1, -1, -1).contiguous() + 0.5
+        b = torch.rand((s, 1, n_ang, n), device=cuda, generator=g) + 0.5
+        pairs.append([engine.BatchedSolver(c, maps, b, method) for _ in range(2)])
+    rag = engine.RaggedSolvers([p[1] for p in pairs])
+    for _ in range(2):
+        rag.step()
+        for p in pairs:
+            p[0].step()
+    for single, ragged in pairs:
+        assert torch.equal(single.x, ragged.x) and torch.equal(single.residuals, ragged.residuals)

@@ -945,8 +945,9 @@ __device__ __forceinline__ float2 bp_lerp2(const float2 (*pairs)[BP_KW], unsigne
 }
 
 // Sum of lines [l0, l1) at the PPT pixels (rows i0 + k, column j) of this thread; ti0, tj0 is the
-// tile's first row and column.
-template <bool SYM, int MAPS_DTYPE, int PPT>
+// tile's first row and column.  ONE: all lines are one chunk and nothing is fetched ahead, which with few lines
+// is most of a CTA's instructions (512^2, 64 slices: 1 line 45 -> 37 us, 4 lines 64 -> 56, 12 lines 103 -> 97).
+template <bool SYM, int MAPS_DTYPE, int PPT, bool ONE>
 __device__ __forceinline__ void bp_segment(const BpArgs& args, BpShared& sh, int s, int ti0, int tj0, int i0, int j,
                                            int l0, int l1, float (&acc)[PPT]) {
   static_assert(PPT % 2 == 0 && BP_LINES <= 32, "pixels go in pairs, lines in one mask");
@@ -1011,8 +1012,8 @@ __device__ __forceinline__ void bp_segment(const BpArgs& args, BpShared& sh, int
 #pragma unroll
     for (int p = 0; p < PER_WARP; ++p) {
       const int ll = warp + (BP_THREADS / 32) * p;
-      const bool in = lc + ll < l1 && sh.line[slot][ll].kind != LINE_EMPTY;
-      const int kk = in ? sh.line[slot][ll].kbase + lane : n;
+      if (lc + ll >= l1) break;
+      const int kk = sh.line[slot][ll].kind != LINE_EMPTY ? sh.line[slot][ll].kbase + lane : n;
       const float* line = sino + (int64_t)(lc + ll) * n;
 #pragma unroll
       for (int q = 0; q < 3; ++q) held[p][q] = (unsigned)(kk + 32 * q) < (unsigned)n ? __ldg(line + kk + 32 * q) : 0.f;
@@ -1040,7 +1041,7 @@ __device__ __forceinline__ void bp_segment(const BpArgs& args, BpShared& sh, int
 
   // (the previous segment's last barrier is behind every thread)
   if (lane < PER_WARP) describe(l0, warp + (BP_THREADS / 32) * lane, 0);
-  if (warp == BP_THREADS / 32 - 1 && lane < BP_LINES) describe(l0 + BP_LINES, lane, 1);
+  if (!ONE && warp == BP_THREADS / 32 - 1 && lane < BP_LINES) describe(l0 + BP_LINES, lane, 1);
   __syncwarp();
   load_chunk(l0, 0);
   store_chunk(l0, 0, 0);
@@ -1048,9 +1049,9 @@ __device__ __forceinline__ void bp_segment(const BpArgs& args, BpShared& sh, int
   int slot = 0, buf = 0;
   for (int lc = l0, c = 0; lc < l1; lc += BP_LINES, buf ^= 1, ++c) {
     const int count = min(BP_LINES, l1 - lc);
-    const bool more = lc + BP_LINES < l1;
+    const bool more = !ONE && lc + BP_LINES < l1;
     const int next = slot == 2 ? 0 : slot + 1;
-    if (warp == (c & 7) && lane < BP_LINES) describe(lc + 2 * BP_LINES, lane, next == 2 ? 0 : next + 1);
+    if (!ONE && warp == (c & 7) && lane < BP_LINES) describe(lc + 2 * BP_LINES, lane, next == 2 ? 0 : next + 1);
     if (!SYM && more) load_chunk(lc + BP_LINES, next);  // SYM keeps the registers for its maps
     const float2 (*pairs)[BP_KW] = sh.pairs[buf];
     const BpLine* lines = sh.line[slot];
@@ -1128,14 +1129,28 @@ __device__ __forceinline__ void bp_segment(const BpArgs& args, BpShared& sh, int
     }
     if (SYM && more) load_chunk(lc + BP_LINES, next);
     if (more) store_chunk(lc + BP_LINES, next, buf ^ 1);
+    if (ONE) break;
     slot = next;
     __syncthreads();
   }
 }
 
+template <int EPI, int PPT>
+__device__ __forceinline__ void bp_epilogue_tile(const BpArgs& args, int s, int i0, int j, const float (&v)[PPT]) {
+  if constexpr (EPI == BP_EPI_MLEM || EPI == BP_EPI_SIRT) {
+    bp_epilogue_rows<EPI, PPT>(args, s, i0, 1, j, v);
+  } else {
+#pragma unroll
+    for (int k = 0; k < PPT; ++k) {
+      const int i = i0 + k;
+      if (i < args.n && j < args.n) bp_epilogue<EPI>(args, s, i, j, v[k]);
+    }
+  }
+}
+
 // One CTA of the back projection: pixel tile `tile` of slice `s`; with CLUSTER, segment `rank` of the
 // cluster's tile, else all segments.
-template <int EPI, bool SYM, int MAPS_DTYPE, int PPT, bool CLUSTER>
+template <int EPI, bool SYM, int MAPS_DTYPE, int PPT, bool CLUSTER, bool ONE>
 __device__ __forceinline__ void bp_tile(const BpArgs& args, BpShared& sh, int tile, int s, int rank, int ranks) {
   constexpr int TI = 8 * PPT;
   const int n = args.n;
@@ -1149,26 +1164,21 @@ __device__ __forceinline__ void bp_tile(const BpArgs& args, BpShared& sh, int ti
   const int n_lines = args.n_det * args.n_angles;
   const int log2_segs = bp_log2_segments(n_lines), segs = 1 << log2_segs;
   float acc[PPT];
-  if constexpr (!CLUSTER) {
+  if constexpr (ONE) {
+    bp_segment<SYM, MAPS_DTYPE, PPT, true>(args, sh, s, ti0, tj0, i0, j, 0, n_lines, acc);
+    bp_epilogue_tile<EPI, PPT>(args, s, i0, j, acc);
+  } else if constexpr (!CLUSTER) {
     float total[PPT];
     for (int g = 0; g < segs; ++g) {
-      bp_segment<SYM, MAPS_DTYPE, PPT>(args, sh, s, ti0, tj0, i0, j, (g * n_lines) >> log2_segs,
+      bp_segment<SYM, MAPS_DTYPE, PPT, false>(args, sh, s, ti0, tj0, i0, j, (g * n_lines) >> log2_segs,
                                        ((g + 1) * n_lines) >> log2_segs, acc);
 #pragma unroll
       for (int k = 0; k < PPT; ++k) total[k] = g == 0 ? acc[k] : total[k] + acc[k];
     }
-    if constexpr (EPI == BP_EPI_MLEM || EPI == BP_EPI_SIRT) {
-      bp_epilogue_rows<EPI, PPT>(args, s, i0, 1, j, total);
-    } else {
-#pragma unroll
-      for (int k = 0; k < PPT; ++k) {
-        const int i = i0 + k;
-        if (i < n && j < n) bp_epilogue<EPI>(args, s, i, j, total[k]);
-      }
-    }
+    bp_epilogue_tile<EPI, PPT>(args, s, i0, j, total);
   } else {
     if (rank < segs) {
-      bp_segment<SYM, MAPS_DTYPE, PPT>(args, sh, s, ti0, tj0, i0, j, (rank * n_lines) >> log2_segs,
+      bp_segment<SYM, MAPS_DTYPE, PPT, false>(args, sh, s, ti0, tj0, i0, j, (rank * n_lines) >> log2_segs,
                                        ((rank + 1) * n_lines) >> log2_segs, acc);
     }
     __syncthreads();
@@ -1189,19 +1199,19 @@ __device__ __forceinline__ void bp_tile(const BpArgs& args, BpShared& sh, int ti
   }
 }
 
-template <int EPI, bool SYM, int MAPS_DTYPE, bool CLUSTER>
+template <int EPI, bool SYM, int MAPS_DTYPE, bool CLUSTER, bool ONE = false>
 __device__ __forceinline__ void bp_cta(const BpArgs& args, int tile, int s, int rank, int ranks) {
   __shared__ __align__(16) BpShared sh;
   if (args.tile_rows == BP_BLOCK_ROWS) {
-    bp_tile<EPI, SYM, MAPS_DTYPE, 8, CLUSTER>(args, sh, tile, s, rank, ranks);
+    bp_tile<EPI, SYM, MAPS_DTYPE, 8, CLUSTER, ONE>(args, sh, tile, s, rank, ranks);
   } else {
-    bp_tile<EPI, SYM, MAPS_DTYPE, 4, CLUSTER>(args, sh, tile, s, rank, ranks);
+    bp_tile<EPI, SYM, MAPS_DTYPE, 4, CLUSTER, ONE>(args, sh, tile, s, rank, ranks);
   }
 }
 
-template <int EPI, bool SYM, int MAPS_DTYPE>
+template <int EPI, bool SYM, int MAPS_DTYPE, bool ONE>
 __global__ void __launch_bounds__(BP_THREADS, 4) bp_kernel(BpArgs args) {
-  bp_cta<EPI, SYM, MAPS_DTYPE, false>(args, blockIdx.x, blockIdx.y, 0, 1);
+  bp_cta<EPI, SYM, MAPS_DTYPE, false, ONE>(args, blockIdx.x, blockIdx.y, 0, 1);
 }
 
 // The same over clusters of `ranks` CTAs along x.
@@ -1523,9 +1533,9 @@ constexpr int64_t BP_FEW_TILES = 352;
 
 // Rows of a batch's tiles (one CTA or, with `segs` > 1, a cluster of as many for each).  A tile of 64 rows
 // stages a line for twice the pixels; tiles of 32 rows pay while their CTAs leave most of the chip idle
-// and a tile's own time counts: up to two per SM in clusters (128^2 x 180: 10.6 us with 32 rows, 11.8 with 64
-// at 1 slice = 128 CTAs, 15.9 and 14.1 at 4 slices = 512), up to four per SM with one segment (192^2 x 4:
-// 6.7 and 7.7 us at 16 slices = 576 CTAs, 10.6 and 9.8 at 32).  Large batches gain most from 64 rows
+// and a tile's own time counts: up to two per SM in clusters (128^2 x 180: 10.8 us with 32 rows, 12.1 with 64
+// at 1 slice = 128 CTAs, 15.5 and 14.3 at 4 slices = 512), up to four per SM with one segment (192^2 x 4:
+// 5.6 and 6.6 us at 16 slices = 576 CTAs, 9.0 and 8.5 at 32).  Large batches gain most from 64 rows
 // (128^2 x 180, 1024 slices: 2020 and 1338 us).
 static int bp_tile_rows(int64_t tiles32, int segs) { return tiles32 * segs <= (segs > 1 ? 296 : 592) ? 32 : BP_BLOCK_ROWS; }
 
@@ -1536,8 +1546,10 @@ static void launch_bp_inst(BpArgs a, cudaStream_t st) {
   const int tiles = bp_tiles(a.n, a.tile_rows);
   if (segs > 1 && (int64_t)tiles * a.n_slices < BP_FEW_TILES) {
     launch_cluster(bp_cluster_kernel<EPI, SYM, MAPS_DTYPE>, dim3(tiles * segs, a.n_slices), segs, st, a, segs);
+  } else if (segs == 1) {  // at most 15 lines
+    bp_kernel<EPI, SYM, MAPS_DTYPE, true><<<dim3(tiles, a.n_slices), BP_THREADS, 0, st>>>(a);
   } else {
-    bp_kernel<EPI, SYM, MAPS_DTYPE><<<dim3(tiles, a.n_slices), BP_THREADS, 0, st>>>(a);
+    bp_kernel<EPI, SYM, MAPS_DTYPE, false><<<dim3(tiles, a.n_slices), BP_THREADS, 0, st>>>(a);
   }
 }
 

@@ -1242,14 +1242,17 @@ __global__ void __launch_bounds__(BP_THREADS, 4) bp_ragged_kernel(const BpArgs* 
 // sqrt(2) < 1.42 of its inverse-rotated lattice position along r and along c: at most three
 // values of each, ceil(position - 1.42) and the next two.
 //
-// Bound: issue (~110 instructions per pixel and line for the nine candidates).  A CTA holds 64 pixels
-// and four threads of each take every fourth line, since one thread per pixel leaves most of the
-// chip's warps empty at 256^2.  Positions and hats are FP32 like the forward's; the products of two
+// Bound: issue (~110 instructions per pixel and line for the nine candidates).  With few pixels a CTA holds 64
+// of them and four threads of each take every fourth line, since one thread per pixel leaves most of the
+// chip's warps empty at 256^2; batches that fill the chip, and a few lines, take one thread per pixel.  Positions and hats are FP32 like the forward's; the products of two
 // hats and all sums are FP64 (253 us; with FP32 products and column sums 230 us, with their errors
 // carried along in FP32 279 us).  256^2 x 360 with 36 candidates per thread and line: 1170 us.
 // ------------------------------------------------------------------------------------------
-constexpr int ADJ_PIXELS = 64;
-constexpr int ADJ_SPLIT = 4;
+constexpr int ADJ_THREADS = 256;
+// Pixels of a batch below which four threads share one: 1.5 waves of CTAs of 256 pixels (256^2 x 60: 40 us
+// with four, 50 with one at 1 slice, 138 and 137 at 4, 588 and 550 at 16), and less for lines that
+// four threads cannot share (256^2 x 1: 5.7 and 4.1 us at 1 slice, 983 and 301 at 256; 128^2 x 3: 4.1 and 5.3).
+constexpr int64_t ADJ_FEW_PIXELS = 227328, ADJ_FEW_LINES_PIXELS = 32768;
 constexpr int ADJ_CHUNK = 32;       // lines whose geometry is staged together
 constexpr float ADJ_REACH = 1.42f;  // > sqrt(2), by more than the FP32 error of the inverse position
 
@@ -1260,15 +1263,16 @@ struct AdjLine {
   int angle, det;
 };
 
-template <bool HAS_MAPS, int MAPS_DTYPE>
-__global__ void __launch_bounds__(ADJ_PIXELS* ADJ_SPLIT) bp_adjoint_kernel(BpArgs args) {
+template <bool HAS_MAPS, int MAPS_DTYPE, int SPLIT>
+__global__ void __launch_bounds__(ADJ_THREADS) bp_adjoint_kernel(BpArgs args) {
+  constexpr int PIXELS = ADJ_THREADS / SPLIT;
   __shared__ AdjLine lines[ADJ_CHUNK];
-  __shared__ double part[ADJ_SPLIT][ADJ_PIXELS];
+  __shared__ double part[SPLIT][PIXELS];
   const int n = args.n;
   const int64_t total = (int64_t)n * n;
   const int s = blockIdx.y;
-  const int tid = threadIdx.x, t = tid % ADJ_PIXELS, g = tid / ADJ_PIXELS;
-  const int64_t pix = (int64_t)blockIdx.x * ADJ_PIXELS + t;
+  const int tid = threadIdx.x, t = tid % PIXELS, g = tid / PIXELS;
+  const int64_t pix = (int64_t)blockIdx.x * PIXELS + t;
   const bool in = pix < total;
   const int pi = in ? (int)(pix / n) : 0, pj = in ? (int)(pix - (int64_t)pi * n) : 0;
   const float fi = (float)pi, fj = (float)pj;
@@ -1298,7 +1302,7 @@ __global__ void __launch_bounds__(ADJ_PIXELS* ADJ_SPLIT) bp_adjoint_kernel(BpArg
       lines[tid] = al;
     }
     __syncthreads();
-    for (int ll = g; in && ll < count; ll += ADJ_SPLIT) {
+    for (int ll = g; in && ll < count; ll += SPLIT) {
       const AdjLine al = lines[ll];
       const float cb = ceilf(fmaf(al.cx, fj, fmaf(al.cy, fi, al.c0)) - ADJ_REACH);
       const float rb = ceilf(fmaf(al.rx, fj, fmaf(al.ry, fi, al.r0)) - ADJ_REACH);
@@ -1337,9 +1341,14 @@ __global__ void __launch_bounds__(ADJ_PIXELS* ADJ_SPLIT) bp_adjoint_kernel(BpArg
       acc += contrib;
     }
   }
-  part[g][t] = acc;
-  __syncthreads();
-  if (g == 0 && in) bp_epilogue<BP_EPI_STORE>(args, s, pi, pj, (float)((part[0][t] + part[1][t]) + (part[2][t] + part[3][t])));
+  if constexpr (SPLIT > 1) {
+    part[g][t] = acc;
+    __syncthreads();
+    acc = 0.0;
+#pragma unroll
+    for (int k = 0; k < SPLIT; k += 2) acc += part[k][t] + part[k + 1][t];
+  }
+  if (g == 0 && in) bp_epilogue<BP_EPI_STORE>(args, s, pi, pj, (float)acc);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1630,17 +1639,28 @@ void launch_bp_ragged(const BpArgs* groups, const int64_t* start, int n_groups, 
   }
 }
 
+template <int SPLIT>
+static void launch_adjoint(const BpArgs& a, cudaStream_t st) {
+  constexpr int pixels = ADJ_THREADS / SPLIT;
+  const dim3 grid((unsigned)(((int64_t)a.n * a.n + pixels - 1) / pixels), a.n_slices);
+  if (a.maps == nullptr) {
+    bp_adjoint_kernel<false, CCT_DTYPE_F32, SPLIT><<<grid, ADJ_THREADS, 0, st>>>(a);
+  } else if (a.maps_dtype == CCT_DTYPE_BF16) {
+    bp_adjoint_kernel<true, CCT_DTYPE_BF16, SPLIT><<<grid, ADJ_THREADS, 0, st>>>(a);
+  } else if (a.maps_dtype == CCT_DTYPE_FIELDS_F32) {
+    bp_adjoint_kernel<true, CCT_DTYPE_FIELDS_F32, SPLIT><<<grid, ADJ_THREADS, 0, st>>>(a);
+  } else {
+    bp_adjoint_kernel<true, CCT_DTYPE_F32, SPLIT><<<grid, ADJ_THREADS, 0, st>>>(a);
+  }
+}
+
 void launch_bp(const BpArgs& a, cudaStream_t st) {
   if (a.mode == CCT_BP_ADJOINT) {
-    const dim3 grid((unsigned)(((int64_t)a.n * a.n + ADJ_PIXELS - 1) / ADJ_PIXELS), a.n_slices);
-    if (a.maps == nullptr) {
-      bp_adjoint_kernel<false, CCT_DTYPE_F32><<<grid, ADJ_PIXELS * ADJ_SPLIT, 0, st>>>(a);
-    } else if (a.maps_dtype == CCT_DTYPE_BF16) {
-      bp_adjoint_kernel<true, CCT_DTYPE_BF16><<<grid, ADJ_PIXELS * ADJ_SPLIT, 0, st>>>(a);
-    } else if (a.maps_dtype == CCT_DTYPE_FIELDS_F32) {
-      bp_adjoint_kernel<true, CCT_DTYPE_FIELDS_F32><<<grid, ADJ_PIXELS * ADJ_SPLIT, 0, st>>>(a);
+    const int64_t pixels = (int64_t)a.n * a.n * a.n_slices;
+    if (pixels < (a.n_det * a.n_angles < 4 ? ADJ_FEW_LINES_PIXELS : ADJ_FEW_PIXELS)) {
+      launch_adjoint<4>(a, st);
     } else {
-      bp_adjoint_kernel<true, CCT_DTYPE_F32><<<grid, ADJ_PIXELS * ADJ_SPLIT, 0, st>>>(a);
+      launch_adjoint<1>(a, st);
     }
     return;
   }

@@ -82,3 +82,24 @@ def test_adjoint_forms_hat_products_in_double(n, angle):
         hy = np.maximum(f(1) - np.abs(_fma32(m11, r, _fma32(m10, f(k), m12)) - axis), f(0)).astype(np.float64)
         want = (hy.T @ hx).astype(f)
         assert np.array_equal(c.bp(y, "adjoint")[0].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("n,n_ang,s", [(33, 1, 31), (33, 3, 31), (64, 3, 8), (33, 4, 208), (33, 4, 209), (64, 37, 57), (130, 5, 14)])
+def test_adjoint_with_one_thread_per_pixel(n, n_ang, s):
+    """Batches on both sides of the rule for the threads of a pixel: the first and the last slice against the
+    scatter definition in FP64."""
+    from oracle import port
+    from pycorrectedemissionct_b200 import core
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    dev = torch.device("cuda", 0)
+    angles = np.linspace(0.2, 2 * np.pi, n_ang, endpoint=False)
+    g = torch.Generator(device=dev).manual_seed(n * s)
+    y = torch.rand((s, 1, n_ang, n), device=dev, generator=g) + 0.5
+    maps = torch.rand((1, n_ang, 1, n, n), device=dev, generator=g).expand(s, -1, -1, -1, -1).contiguous()
+    got = core.XrfCore(n, angles, device=dev).bp(y, "adjoint", maps).double().cpu().numpy()
+    _, deg32 = port.backend_angles(angles)
+    for k in (0, s - 1):
+        ref = port.fp_xrf_adjoint(y[k].double().cpu().numpy(), maps[k].double().cpu().numpy(), deg32, n)
+        assert rel_l2(got[k], ref) < TOL

@@ -171,7 +171,7 @@ int cct_maps_workspace_size(const cct_maps_desc* desc, int32_t angles_per_pass, 
    angles per pass is the largest that fits in workspace_bytes.  When the workspace also holds
    copies of mu_in and of a distinct mu_out beside at least half of that many entries, its start
    holds those copies (rows of `pitch` = n rounded up to 4 floats; n * pitch * S floats each,
-   256-byte rounded): transposed ones, which the column scans read at angles whose columns run
+   256-byte rounded; none for sets so small that they do not pay): transposed ones, which the column scans read at angles whose columns run
    closer to y than to x, and where n % 4 != 0 row-major ones too (same results, wider loads).
    maps_dtype = CCT_DTYPE_FIELDS_F32
    writes the line-integral fields [S][A][1 + D][n][n] (L_in, then L_out per detector; zero for an

@@ -400,6 +400,8 @@ def compute_maps(
     need = int(size.value)
     own_out = mu_out is not None and not use_quads and (mu_in is None or mu_out.data_ptr() != mu_in.data_ptr())
     copies = (int(mu_in is not None) + int(own_out)) * _maps_copy_bytes(n, s)
+    if n < 128 and need // 4 * entries < 262144:  # the library scans such sets in place
+        copies = 0
     if workspace is None:
         # beside the copies of mu, at least 8 angles (of the whole batch) per pass, at most all of them
         nbytes = min(max(int(workspace_bytes), 8 * need + copies), need * entries + copies)

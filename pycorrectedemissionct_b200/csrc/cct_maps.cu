@@ -665,11 +665,18 @@ static void launch_copies(const cct_maps_desc* d, const float* mu, char** work, 
   }
 }
 
+// Copies take two or four launches of ~2 us each, which small sets do not repay: one angle of 33^2 x 4 slices
+// 16.4 us (40 with the host's launches) with copies and 11.9 (29) in place, 16 angles of 64^2 18.4 (37) and 20.1
+// (31), one angle of 128^2 19.2 (35) and 29.1 (33), of 256^2 26.6 and 50.
+constexpr int COPIES_PAY_N = 128;
+constexpr int64_t COPIES_PAY_ELEMENTS = 262144;  // of W, over all entries
+
 // Entries per pass and whether the workspace also holds the copies of `volumes` attenuation volumes at
 // its start: they are used when, after them, at least half the entries of a pass without them fit.
 static int plan_pass(const cct_maps_desc* d, size_t work_bytes, int64_t per_entry, int entries, int volumes,
                      size_t* prefix) {
-  const int copies = volumes * (copy_pitch(d->n) != d->n ? 2 : 1);
+  const bool pay = d->n >= COPIES_PAY_N || per_entry / (int64_t)sizeof(float) * entries >= COPIES_PAY_ELEMENTS;
+  const int copies = pay ? volumes * (copy_pitch(d->n) != d->n ? 2 : 1) : 0;
   const int64_t plain = std::min<int64_t>((int64_t)work_bytes / per_entry, entries);
   const size_t tb = (size_t)copies * copy_bytes(d);
   const int64_t with_t = work_bytes > tb ? std::min<int64_t>((int64_t)(work_bytes - tb) / per_entry, entries) : 0;

@@ -41,7 +41,7 @@ def test_maps_passes_and_copies(n, n_ang, quads):
     ref, scans = _scans(lambda: core.compute_maps(*args))
     assert core.compute_maps.last_passes == 1 and scans in (1, None)
     need = core.maps_entry_bytes(n, s)
-    copies = 2 * core._maps_copy_bytes(n, s)
+    copies = 2 * core._maps_copy_bytes(n, s)  # (sides of 33 and 64 with few angles take none)
     # one entry in place (narrow loads where n % 4 != 0), one and three beside the copies, and between
     for nbytes in (need, need + copies // 2, need + copies, 3 * need + copies - 4, 3 * need + copies):
         ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")

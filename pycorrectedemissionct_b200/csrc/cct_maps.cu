@@ -165,7 +165,7 @@ __device__ __forceinline__ void column_support(double ax, double bx, double ay, 
 // Scan
 //
 // A CTA owns 64 rotated-frame columns of one job and walks their support rows in chunks of 64.  The
-// bounding box of a chunk in mu (at most 94 x 100 pixels, zeros outside the image) is staged in
+// bounding box of a chunk in mu (at most 94 rows of 103 pixels, zeros outside the image) is staged in
 // shared memory; each of 256 threads then samples 16 consecutive rows of one column, the column's four
 // threads exchange their FP64 sums, and each writes its rows.  A warp is 32 neighbouring columns at
 // one row, so the stores of W are coalesced; where the columns run closer to y than to x the box comes

@@ -55,18 +55,10 @@ static_assert(FP_MAX_CHUNKS <= FP_THREADS, "one thread per chunk box");
 constexpr int FP_FILL_BATCH = 3;                   // float4 items whose loads are issued together
 
 template <bool HAS_MAPS, int MAPS_DTYPE>
-__device__ __forceinline__ float4 fp_load_item(const float* vol, const MapRef& mref, int n, int gy, int gx, bool vec4) {
+__device__ __forceinline__ float4 fp_load_item(const float* vol, const MapRef& mref, int n, int gy, int gx) {
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
   if (gy < 0 || gy >= n || gx + 3 < 0 || gx >= n) return v;
   const int off = gy * n + gx;  // < 2^31 for n <= 8192... n*n <= 2^26
-  if (vec4 && gx >= 0 && gx + 3 < n) {
-    v = __ldg(reinterpret_cast<const float4*>(vol + off));
-    if (HAS_MAPS) {
-      const float4 mv = map_at4<MAPS_DTYPE>(mref, off);
-      v.x *= mv.x; v.y *= mv.y; v.z *= mv.z; v.w *= mv.w;
-    }
-    return v;
-  }
   float e[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
@@ -170,7 +162,9 @@ __device__ __forceinline__ void fp_write_partial(double v, double* partials, int
 template <int DT>
 __device__ __forceinline__ void fp_prefetch_rows(const MapRef& m, int n, const int4 box, int tid) {
   constexpr int ES = DT == CCT_DTYPE_BF16 ? 2 : 4;
-  constexpr int LINES = DT == CCT_DTYPE_BF16 ? 2 : 4;  // lines of a row (of at most 400 bytes and where it begins in its first line)
+  // lines asked for of a row, which has at most 400 (BF16: 200) bytes: the end of a row that reaches into one
+  // more line (BF16 rows near 45 degrees, FP32 rows at n % 4 != 0) is left to the fill
+  constexpr int LINES = DT == CCT_DTYPE_BF16 ? 2 : 4;
   const int x0 = max(box.x, 0), x1 = min(box.y + 1, n);
   const int line = tid % LINES;
 #pragma unroll
@@ -293,7 +287,7 @@ __device__ __forceinline__ void fp_cta(const FpArgs& args, const int band, const
               }
             }
           } else {
-            v[k] = fp_load_item<HAS_MAPS, MAPS_DTYPE>(vol, mref, n, gy, gx, false);
+            v[k] = fp_load_item<HAS_MAPS, MAPS_DTYPE>(vol, mref, n, gy, gx);
           }
         }
       }
@@ -646,7 +640,7 @@ __device__ __forceinline__ float4 fp2_quad(const float* vol, const MapRef& mref,
     }
     return v;
   }
-  return fp_load_item<HAS_MAPS, MAPS_DTYPE>(vol, mref, n, gy, gx, false);
+  return fp_load_item<HAS_MAPS, MAPS_DTYPE>(vol, mref, n, gy, gx);
 }
 
 template <int EPI, bool HAS_MAPS, int MAPS_DTYPE>

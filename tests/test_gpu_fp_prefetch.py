@@ -44,3 +44,10 @@ def test_fields_fill_leaves_out_only_unread_quads(n, channels):
         c.fp(torch.full_like(x, 1e30), fields)
         out.append(c.fp(x, fields))
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("n,channels", [(2, 2), (3, 2), (3, 4), (5, 2)])
+def test_fields_fill_of_the_smallest_sides(n, channels):
+    """The same with two channels at least: the two-slice kernel takes pairs only, and one slice goes to the
+    plain kernel itself."""
+    test_fields_fill_leaves_out_only_unread_quads(n, channels)

@@ -843,8 +843,9 @@ __global__ void __launch_bounds__(FP_THREADS, 4) fp_pair_kernel(FpArgs args) {
 // the time went on was the rare case: the FP64 edge decision, inlined per pixel or called, cost
 // registers and branches on every line (1.20 ms with the call, 0.99 ms with no edge at all, 1.13 ms
 // as below, for 16 slices), and the three barriers per chunk of lines.  Measured on 512^2 x 720
-// (start -> now): 1 slice 281 -> 106 us, 8 slices 880 -> 597 us, 16 slices 1519 -> 1128 us; 256^2 x
-// 360 161 -> 23 us, 128^2 x 180 77 -> 11 us; with maps (512^2 x 360, 2 slices) 1577 -> 278 us.
+// (before -> now): 1 slice 281 -> 99 us, 8 slices 880 -> 621 us, 16 slices 1519 -> 1134 us; 256^2 x
+// 360 161 -> 23 us, 128^2 x 180 77 -> 11 us; with maps (512^2 x 360, 2 slices) 1577 -> 278 us.  (Values at
+// the edges in FP64 cost four spilled registers where one CTA walks all segments: 8 slices 600 us without.)
 //
 // The lines are summed in up to eight fixed segments, whose sums are added in order (which also
 // shortens the FP32 sums: the error against FP64 falls from 3.9e-7 to 1e-7 at 722 lines).  One CTA
